@@ -191,6 +191,7 @@ __device__ __forceinline__ Ctx make_ctx(unsigned char *smem, const ClusterLayout
     t.OV = (uint32_t *)(smem + ly.off_OV);
     t.FLIP = (uint32_t *)(smem + ly.off_FLIP);
     t.ROOT = (uint32_t *)(smem + ly.off_ROOT);
+    t.NEED = t.ROOT;  // read by the unions, before the roots are recorded
     t.RE = nullptr;
     t.SEAMV = nullptr;
     t.wrap = &red.wrap;
@@ -456,9 +457,10 @@ __device__ __forceinline__ uint32_t node_key(uint32_t hk) { return hk & 0xFFFFu;
 // cluster kernel keeps more state live across its phases than the resident
 // one, and compiled inline these pointer-chasing loops lose registers to it.
 template <int NT>
-static __device__ __noinline__ void cluster_union(const Lat<Word16> &t, uint32_t tid)
+static __device__ __noinline__ void cluster_union(const Lat<Word16> &t, unsigned short *list, uint32_t seg,
+                                                  uint32_t warp)
 {
-    phase_union_open(t, tid, NT);
+    phase_union_open<false>(t, list, seg, warp, NT / 32);
 }
 
 template <int NT>
@@ -549,20 +551,23 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             tile_activate<NT>(x.t, x.YS, tl, make_rng(ch.key, sweep, ch.thr), gJH, gJV, front, red.tile_end, warp,
                               nwarps, tid);
             __syncthreads();
-            phase_heads<Word16>(t, warp, nwarps);
-            for (uint32_t w = tid; w < t.g.NW; w += NT) t.ROOT[w] = 0u;
-            for (uint32_t k = tid; k < x.hs; k += NT) {
-                x.HK[k] = kEmptyKey;
-                x.HW[k] = Word64::make((c << 16) | k, 0, 0);
-            }
+            phase_heads_open<false>(t, warp, nwarps);
+            for (uint32_t k = tid; k < x.hs; k += NT) x.HK[k] = kEmptyKey;
             __syncthreads();
-            cluster_union<NT>(t, tid);
+            // The warp's union list lies in its share of the node words, which
+            // are reset afterwards.
+            const uint32_t share = x.hs / nwarps;
+            cluster_union<NT>(t, (unsigned short *)(x.HW + warp * share), 4u * share, warp);
+            for (uint32_t k = warp * share + lane; k < (warp + 1u) * share; k += 32u)
+                x.HW[k] = Word64::make((c << 16) | k, 0, 0);
             __syncthreads();
             // With at least one word per thread the roots are found in one
             // pass with the flip, after the boundary stage (roots_flip_pieces);
             // the boundary bonds' tile roots are then found by read-only walks.
             const bool merged = t.g.NW >= (uint32_t)NT;
             if (!merged) {
+                for (uint32_t w = tid; w < t.g.NW; w += NT) t.ROOT[w] = 0u;
+                __syncthreads();
                 cluster_roots<NT>(t, tid);
                 __syncthreads();
             }

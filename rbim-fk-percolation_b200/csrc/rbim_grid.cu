@@ -86,7 +86,7 @@ __host__ __device__ constexpr size_t g256(size_t v) { return (v + 255) & ~size_t
 // Shared-memory layout of one CTA's tile for an L x L lattice split in C
 // tiles.
 struct GridLayout {
-    uint32_t L, C, t_max, tw, rows_max, node_max, bh;
+    uint32_t L, C, t_max, tw, rows_max, node_max, bh, list;
     size_t off_uf, off_S, off_OH, off_OV, off_FLIP, off_ROOT, off_NODE, off_YS, off_NK, off_NR, off_BH, bytes;
 };
 
@@ -125,6 +125,10 @@ GridLayout grid_layout(uint32_t L, uint32_t C, bool with_hash)
     off = g16(off + 4ull * ly.node_max);
     ly.off_NR = off;  // node list: root node (global site) after the boundary stage
     off = g16(off + 4ull * ly.node_max);
+    // The node lists' memory also holds the warps' union lists: at least 32
+    // 16-bit entries for each of up to 32 warps.
+    off = std::max(off, ly.off_NK + 2048u);
+    ly.list = (uint32_t)(off - ly.off_NK) / 2u;
     ly.bh = 0;
     if (with_hash) {
         const uint32_t items = L + 1u + ly.rows_max;
@@ -394,6 +398,7 @@ __device__ __forceinline__ GTile make_gtile(unsigned char *smem, const GridLayou
     t.err = &red.err;
     t.cap = cap;
     x.NODE = (uint32_t *)(smem + ly.off_NODE);
+    t.NEED = x.NODE;  // read by the unions, before the nodes are listed
     x.YS = (uint32_t *)(smem + ly.off_YS);
     x.NK = (uint32_t *)(smem + ly.off_NK);
     x.NR = (uint32_t *)(smem + ly.off_NR);
@@ -571,9 +576,10 @@ __device__ __forceinline__ void grid_boundary(const GTile &x, const Tile &tl, co
 // in the cluster engine: inline, these pointer-chasing loops lose registers
 // to the state the kernel keeps live across its phases.
 template <int NT>
-static __device__ __noinline__ void grid_union(const Lat<Word16> &t, uint32_t tid)
+static __device__ __noinline__ void grid_union(const Lat<Word16> &t, unsigned short *list, uint32_t seg,
+                                               uint32_t warp)
 {
-    phase_union_open(t, tid, NT);
+    phase_union_open<true>(t, list, seg, warp, NT / 32);
 }
 
 template <int NT>
@@ -731,7 +737,6 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
             red.nnodes = 0;
         }
         for (uint32_t i = tid; i < ly.rows_max / 32u + 1u; i += NT) x.YS[i] = 0u;
-        for (uint32_t w = tid; w < t.g.NW; w += NT) x.NODE[w] = 0u;
         for (uint32_t i = tid; i < ly.bh; i += NT) x.BH[i] = ~0ull;
         __syncthreads();
         tile_activate<NT>(t, x.YS, tl, make_rng(ch.key, sweep, ch.thr), gJH, gJV, front, red.tile_end, warp, nwarps,
@@ -739,14 +744,16 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
         __syncthreads();
         RBIM_GRID_MARK(0);
         for (uint32_t w = tid; w < t.g.NW; w += NT) ws.FLIPG[(tl.b >> 5) + w] = t.FLIP[w];
-        phase_heads<Word16>(t, warp, nwarps);
+        phase_heads_open<true>(t, warp, nwarps);
         for (uint32_t w = tid; w < t.g.NW; w += NT) t.ROOT[w] = 0u;
         __syncthreads();
         RBIM_GRID_MARK(1);
-        grid_union<NT>(t, tid);
+        const uint32_t seg = ly.list / nwarps;  // union lists, in the node lists' memory
+        grid_union<NT>(t, (unsigned short *)x.NK + warp * seg, seg, warp);
         __syncthreads();
         RBIM_GRID_MARK(2);
         grid_roots<NT>(t, tid);
+        for (uint32_t w = tid; w < t.g.NW; w += NT) x.NODE[w] = 0u;
         __syncthreads();
         RBIM_GRID_MARK(3);
         grid_nodes<NT>(x, tl, ws, red, tid);

@@ -12,9 +12,9 @@ namespace rbim {
 // Shared-memory layout of the resident engine for lattices of up to n_max
 // sites (n_max <= 65536).
 struct ResidentLayout {
-    uint32_t n_max, nw_max, l_max, hs;
+    uint32_t n_max, nw_max, l_max, hs, seg;
     size_t off_uf, off_S, off_JH, off_JV, off_OH, off_OV, off_FLIP, off_ROOT, off_RE, off_SEAMV, off_HK, off_HW,
-        bytes;
+        off_LIST, bytes;
 };
 
 ResidentLayout resident_layout(uint32_t l_max, int threads);

@@ -58,44 +58,180 @@ struct UF<Word16> {
     {
         asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(sa + 2u * i), "r"(v) : "memory");
     }
-    __device__ __forceinline__ T cas(uint32_t i, T expect, T v) const
+    // Hooks root hi under lo; false when hi is no longer a root, or when the
+    // other parent in its 32-bit word changed meanwhile.
+    __device__ __forceinline__ bool hook(uint32_t hi, uint32_t lo) const
     {
-        T old;
-        asm volatile("atom.shared.cas.b16 %0, [%1], %2, %3;"
-                     : "=h"(old)
-                     : "r"(sa + 2u * i), "h"(expect), "h"(v)
+        const uint32_t at = (sa + 2u * hi) & ~3u, sh = 16u * (hi & 1u);
+        uint32_t cur, old;
+        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(cur) : "r"(at) : "memory");
+        if (((cur >> sh) & 0xFFFFu) != hi) return false;
+        asm volatile("atom.shared.cas.b32 %0, [%1], %2, %3;"
+                     : "=r"(old)
+                     : "r"(at), "r"(cur), "r"(cur ^ ((hi ^ lo) << sh))
                      : "memory");
-        return old;
+        return old == cur;
     }
     __device__ __forceinline__ void add(uint32_t i, T v) const { uf_atomic_add(w + i, v); }
 };
 
-// Mask of the bits of word w whose site lies in the last row (x = L-1): the
-// horizontal bonds there close the x boundary.
-__device__ __forceinline__ uint32_t last_row_mask(const Geom &g, uint32_t w)
-{
-    const uint32_t n0 = w << 5, first = g.N - g.L;
-    if (n0 + 32u <= first) return 0u;
-    const uint32_t v = g.valid(w);
-    if (n0 >= first) return v;
-    return ~((1u << (first - n0)) - 1u) & v;
-}
+// Bits reached by filling upwards from the seeds s (a subset of p) through
+// consecutive bits of p: adding a seed to its run of ones carries through the
+// run's end, and the carry clears the bits it passes.
+__device__ __forceinline__ uint32_t fill_up(uint32_t s, uint32_t p) { return p & (~(p + s) | s); }
 
-// Occupied x-bonds of word w that need a union: off the x seam, and not
-// already connected through an elementary plaquette with the bond before.
-__device__ __forceinline__ uint32_t union_need(const Lat<Word16> &t, uint32_t w)
+// The up-bonds of word w (bit b: the x-bond from site n - L to n = 32w + b)
+// that the labelling needs, split in links and unions.
+struct UpBonds {
+    uint32_t heads;   // run heads of the word
+    uint32_t above;   // run heads of the sites n - L
+    uint32_t link;    // bonds that link their run's head to the run above
+    uint32_t need;    // bonds left to the unions
+};
+
+__device__ __forceinline__ UpBonds up_bonds(const Lat<Word16> &t, uint32_t w)
 {
     const Geom &g = t.g;
-    const uint32_t oh = t.OH[w] & ~last_row_mask(g, w);
-    if (!oh) return 0u;
-    Plane OVp{t.OV};
-    const uint32_t ohp = w ? t.OH[w - 1u] : 0u;
-    const uint32_t ov = OVp(w), ovp = w ? OVp(w - 1u) : 0u;
-    const uint32_t prev_oh = (oh << 1) | (ohp >> 31);
-    const uint32_t prev_ov = (ov << 1) | (ovp >> 31);
-    uint32_t s = (w << 5) + g.L - 1u;
-    if (s >= g.N) s -= g.N;
-    return oh & ~(prev_oh & prev_ov & extract32(OVp, s, g));
+    UpBonds r;
+    const uint32_t valid = g.valid(w);
+    r.heads = head_mask(t.OV, w, valid);
+    r.above = 0u;
+    r.link = 0u;
+    r.need = 0u;
+    if ((w << 5) + 31u < g.L) return r;  // the first row has no up-bonds
+    // Bits u - 1 .. u + 31 of OH and u - 1 .. u + 30 of OV (words before the
+    // planes read as zero), u = 32w - L the site above bit 0.
+    const int u = (int)(w << 5) - (int)g.L, q = u - 1;
+    const int qw = q >> 5;
+    const uint32_t sh = (uint32_t)q & 31u;
+    const uint32_t h0 = qw >= 0 ? t.OH[qw] : 0u, h1 = t.OH[qw + 1];
+    const uint32_t v0 = qw >= 0 ? t.OV[qw] : 0u, v1 = t.OV[qw + 1];
+    const uint32_t up1 = __funnelshift_r(h0, h1, sh);  // bit 0: the up-bond of the site before the word
+    const uint32_t up = ((up1 >> 1) | ((h1 >> sh) << 31)) & valid;
+    r.above = ~__funnelshift_r(v0, v1, sh);
+    // One bond per pair of runs: a bond is redundant after another one between
+    // the same two runs (no head of either row between them).
+    const uint32_t p = ~(r.heads | r.above);
+    const uint32_t c = up & ~fill_up(((up << 1) | (up1 & 1u)) & p, p);
+    // The first bond of each run headed in this word whose upper run's head is
+    // also in view links the two heads.
+    const uint32_t k = c & (r.heads | (0u - r.heads)) & (r.above | (0u - r.above));
+    const uint32_t in_run = ~r.heads;
+    r.link = k & ~fill_up((k << 1) & in_run, in_run);
+    r.need = c & ~r.link;
+    return r;
+}
+
+// Words of the band of a warp: the words are split in equal contiguous bands,
+// one per warp.
+struct Band {
+    uint32_t first, end;
+};
+
+__device__ __forceinline__ Band warp_band(uint32_t NW, uint32_t warp, uint32_t nwarps)
+{
+    const uint32_t per = (NW + nwarps - 1u) / nwarps;
+    const uint32_t first = min(NW, warp * per);
+    return {first, min(NW, first + per)};
+}
+
+// Parent of one site of a word: the last run head up to it (`le`: the bits up
+// to the site's), or for a head whose run has a link the head above the link,
+// or that head's own parent when it was written before (`done` sites from
+// band0 on).  h, link, above: the word's UpBonds; before: 1 + the last head
+// before the word; n0: the word's first site.
+__device__ __forceinline__ uint32_t open_parent(const UF<Word16> &uf, uint32_t h, uint32_t before, uint32_t link,
+                                                uint32_t above, uint32_t n0, uint32_t le, uint32_t L, uint32_t band0,
+                                                uint32_t done)
+{
+    const uint32_t f = link & ~(le >> 1);  // the lowest of f is the link of a run headed here ...
+    const uint32_t upto = f ^ (f - 1u);
+    const bool linked = f && (h & (le ^ (le >> 1))) && !(h & upto & ~le);  // ... if no other head comes before
+    const uint32_t m = linked ? above & upto : h & le;
+    uint32_t p = (linked ? n0 - L : n0) + 31u - __clz(m);
+    if (!m) p = before - 1u;
+    if (linked && p - band0 < done) p = uf.ld(p);
+    return p;
+}
+
+// 1 + the last run head before word w (0: there is none).
+__device__ __forceinline__ uint32_t last_head_before(const Lat<Word16> &t, uint32_t w)
+{
+    // Site 0 always heads a run, so this walk back ends.
+    while (w-- > 0) {
+        const uint32_t h = head_mask(t.OV, w, 0xFFFFFFFFu);
+        if (h) return (w << 5) + 32u - __clz(h);
+    }
+    return 0u;
+}
+
+// (b) Union-find initialisation: every site points at the head of its run of
+// occupied y-bonds, and a run head with an occupied x-bond to the row above at
+// the run above, with plain stores (a head takes one such link, to a smaller
+// site, so nothing can race).  A warp writes its band of consecutive words two
+// by two (lanes 0-15 one word, 16-31 the next, two sites a lane, one 32-bit
+// store; sites past N are not written); a link whose upper head was written in
+// an earlier step takes that head's own parent, so inside a band the link
+// trees stay one level deep, and a link into the band above (written by
+// another warp meanwhile) takes the upper head itself.  The bonds that are
+// left go to NEED for the unions: at L = 256 about 9 k of 28 k bonds.
+//
+// Per group of 32 words, lane j finds the heads and up-bonds of word j, and a
+// max-scan over the lanes gives every word the last head before it.  kFew: for
+// launches whose warps may have a single word, which all lanes then look at.
+template <bool kFew>
+__device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t warp, uint32_t nwarps)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const Geom &g = t.g;
+    const Band band = warp_band(g.NW, warp, nwarps);
+    if (kFew && band.end - band.first == 1u) {
+        const uint32_t w = band.first, n0 = w << 5;
+        const UpBonds ub = up_bonds(t, w);
+        if (lane == 0) t.NEED[w] = ub.need;
+        const uint32_t before = (ub.heads & 1u) ? 0u : last_head_before(t, w);
+        const uint32_t p = open_parent(t.uf, ub.heads, before, ub.link, ub.above, n0, mask_le(lane), g.L, 0u, 0u);
+        if (n0 + lane < g.N) t.uf.st(n0 + lane, (unsigned short)p);
+        return;
+    }
+    const uint32_t band0 = band.first << 5, b0 = 2u * (lane & 15u), le0 = mask_le(b0);
+    for (uint32_t base = band.first; base < band.end; base += 32u) {
+        const uint32_t wj = base + lane;
+        UpBonds ub{};
+        if (wj < band.end) {
+            ub = up_bonds(t, wj);
+            t.NEED[wj] = ub.need;
+        }
+        const uint32_t h = ub.heads;
+        const uint32_t pre = lane == 0 && !(h & 1u) ? last_head_before(t, base) : 0u;
+        const uint32_t count = min(32u, band.end - base);
+        uint32_t incl = max(h ? (wj << 5) + 32u - __clz(h) : 0u, pre);
+        for (uint32_t o = 1; o < count; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl = max(incl, v);
+        }
+        // Last head before word j: the scan of lanes < j, or pre for j = 0.
+        uint32_t before = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
+        if (lane == 0) before = pre;
+        for (uint32_t j = 0; j < count; j += 2u) {
+            const uint32_t jj = j + (lane >> 4);
+            const uint32_t hj = __shfl_sync(0xFFFFFFFFu, h, jj);
+            const uint32_t cj = __shfl_sync(0xFFFFFFFFu, before, jj);
+            const uint32_t lj = __shfl_sync(0xFFFFFFFFu, ub.link, jj);
+            const uint32_t aj = __shfl_sync(0xFFFFFFFFu, ub.above, jj);
+            const uint32_t n0 = (base + jj) << 5, n = n0 + b0;
+            const uint32_t done = ((base + j) << 5) - band0;  // sites of the band written in earlier steps
+            const uint32_t p0 = open_parent(t.uf, hj, cj, lj, aj, n0, le0, g.L, band0, done);
+            const uint32_t p1 = open_parent(t.uf, hj, cj, lj, aj, n0, 2u * le0 + 1u, g.L, band0, done);
+            if (jj < count) {
+                if (n + 1u < g.N)
+                    t.uf.st2(n, p0 | (p1 << 16));
+                else if (n < g.N)
+                    t.uf.st(n, (unsigned short)p0);
+            }
+            __syncwarp();  // later rows read these words
+        }
+    }
 }
 
 // One path-halving step of a walk at x, without branches: returns the next
@@ -111,53 +247,104 @@ __device__ __forceinline__ uint32_t halving_step(const UF<Word16> &uf, uint32_t 
     return x_root ? x : (p_root ? p : gp);
 }
 
-// (b) Open-lattice unions across occupied x-bonds that do not cross the x
-// seam: the larger root is hooked under the smaller with a 16-bit CAS, finds
-// use path halving, and a union whose CAS loses a race restarts from the two
-// roots it found.  Both endpoint walks advance in the same loop iteration.
-__device__ __forceinline__ void phase_union_open(const Lat<Word16> &t, uint32_t tid, uint32_t nthreads)
+// Lists the set bits of a group of `count` words (lane j holds what is left of
+// word j in `bits`) in the warp's `list` of `seg` entries, in order, an entry
+// being 32 j + bit; the bits listed are cleared.  Returns the number of
+// entries.  kFew: up to eight words are listed bit by lane.
+template <bool kFew>
+__device__ __forceinline__ uint32_t list_bits(uint32_t &bits, uint32_t count, unsigned short *list, uint32_t seg,
+                                              uint32_t lane)
+{
+    uint32_t total = 0;
+    if (kFew && count <= 8u) {
+        for (uint32_t j = 0; j < count; ++j) {
+            const uint32_t b = __shfl_sync(0xFFFFFFFFu, bits, j);
+            const uint32_t k = total + __popc(b & (mask_le(lane) >> 1));
+            const bool put = ((b >> lane) & 1u) && k < seg;
+            if (put) list[k] = (unsigned short)((j << 5) + lane);
+            const uint32_t left = b & ~__ballot_sync(0xFFFFFFFFu, put);
+            if (lane == j) bits = left;
+            total += __popc(b);
+        }
+        total = min(total, seg);
+    } else {
+        const uint32_t mine = __popc(bits);
+        uint32_t sum = mine;
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        for (uint32_t k = sum - mine; bits && k < seg; ++k) {
+            list[k] = (unsigned short)((lane << 5) + __ffs(bits) - 1u);
+            bits &= bits - 1u;
+        }
+        total = min(__shfl_sync(0xFFFFFFFFu, sum, 31), seg);
+    }
+    __syncwarp();
+    return total;
+}
+
+// (b) Open-lattice unions across the x-bonds that phase_heads_open left in
+// NEED: the larger root is hooked under the smaller with a CAS, finds use path
+// halving, and a union whose CAS loses a race goes on from the two roots it
+// found.  Bonds per word vary, so each warp lists the bonds of 32 words at a
+// time and its lanes then take every 32nd of them, in one flat loop: both walks of a bond advance in the same iteration and a lane takes its next bond
+// as soon as its union is done.  The CAS works on the 32-bit word that holds
+// the root's parent; losing it to a change of the other half only repeats it.
+//
+// kFew: for launches whose warps may have few words (one lattice or tile on
+// many threads), which are listed at once; the code for it costs 4 % at
+// L = 64 where it is never taken.
+template <bool kFew>
+__device__ __forceinline__ void phase_union_open(const Lat<Word16> &t, unsigned short *list, uint32_t seg,
+                                                 uint32_t warp, uint32_t nwarps)
 {
     const Geom &g = t.g;
     const UF<Word16> &uf = t.uf;
-    const Slices sl = make_slices(g.NW, nthreads);
-    uint32_t item = tid, pending = 0, base = 0;
-    uint32_t xa = 0, xb = 0;
-    bool fetch = true;
+    const uint32_t lane = threadIdx.x & 31u;
+    const Band band = warp_band(g.NW, warp, nwarps);
     const uint32_t cap = 64u * t.cap;  // 64 walks of t.cap steps (64 N + 4096 by default)
     uint32_t it = 0;
     RBIM_PROF_ONLY(uint32_t n_bonds = 0; uint32_t n_fails = 0);
-    for (;; ++it) {
-        if (it >= cap) {
-            atomicOr(t.err, kErrUnionCap);
-            break;
-        }
-        if (fetch) {
-            while (!pending && item < sl.items) {
-                const uint32_t w = sl.word(item);
-                pending = union_need(t, w) & sl.mask(item);
-                base = w << 5;
-                item += nthreads;
-            }
-            if (!pending) break;
-            xa = base + (uint32_t)(__ffs(pending) - 1);
-            pending &= pending - 1u;
-            xb = xa + g.L;
-            fetch = false;
-            RBIM_PROF_ONLY(++n_bonds);
-        }
-        bool da, db;
-        xa = halving_step(uf, xa, da);
-        xb = halving_step(uf, xb, db);
-        if (da && db) {
-            // Both walks are at roots.
-            if (xa == xb) {
-                fetch = true;
+    for (uint32_t base = band.first; base < band.end; base += 32u) {
+        const uint32_t count = min(32u, band.end - base);
+        uint32_t pend = lane < count ? t.NEED[base + lane] : 0u;
+        while (__any_sync(0xFFFFFFFFu, pend != 0u)) {
+            // The bonds of a single word need no list: lane b takes bit b.
+            const bool one = kFew && count == 1u;
+            uint32_t total;
+            if (one) {
+                total = (__shfl_sync(0xFFFFFFFFu, pend, 0) >> lane) & 1u ? lane + 1u : 0u;
+                pend = 0u;
             } else {
-                const uint32_t lo = min(xa, xb), hi = max(xa, xb);
-                fetch = uf.cas(hi, (unsigned short)hi, (unsigned short)lo) == (unsigned short)hi;
-                // A lost race leaves both walks at their old roots, to resume from.
-                RBIM_PROF_ONLY(n_fails += fetch ? 0u : 1u);
+                total = list_bits<kFew>(pend, count, list, seg, lane);
             }
+            uint32_t xa = 0, xb = 0;
+            bool fetch = true;
+            for (uint32_t i = lane;; ++it) {
+                if (fetch) {
+                    if (i >= total) break;
+                    xb = (base << 5) + (one ? lane : (uint32_t)list[i]);
+                    xa = xb - g.L;
+                    i += 32u;
+                    fetch = false;
+                    RBIM_PROF_ONLY(++n_bonds);
+                }
+                if (it >= cap) {
+                    atomicOr(t.err, kErrUnionCap);
+                    break;
+                }
+                bool da, db;
+                xa = halving_step(uf, xa, da);
+                xb = halving_step(uf, xb, db);
+                if (da && db) {
+                    // Both walks are at roots.
+                    fetch = xa == xb || uf.hook(max(xa, xb), min(xa, xb));
+                    RBIM_PROF_ONLY(n_fails += fetch ? 0u : 1u);
+                }
+            }
+            __syncwarp();
         }
     }
 #ifdef RBIM_PROFILE_PHASES
@@ -172,7 +359,7 @@ __device__ __forceinline__ void phase_union_open(const Lat<Word16> &t, uint32_t 
             nb += __shfl_xor_sync(0xFFFFFFFFu, nb, o);
             nf += __shfl_xor_sync(0xFFFFFFFFu, nf, o);
         }
-        if ((threadIdx.x & 31u) == 0) {
+        if (lane == 0) {
             RBIM_COUNT(3, mx);
             RBIM_COUNT(4, sm);
             RBIM_COUNT(0, nb);

@@ -97,7 +97,7 @@ struct SeamWord {
 // Shared-memory layout for lattices of up to l_max x l_max sites; constexpr so
 // that the launches of the common size classes get it as a compile-time
 // constant (the kernel's shared-memory views then need no registers).
-__host__ __device__ constexpr ResidentLayout resident_layout_c(uint32_t l_max)
+__host__ __device__ constexpr ResidentLayout resident_layout_c(uint32_t l_max, int threads)
 {
     ResidentLayout ly{};
     ly.l_max = l_max;
@@ -131,15 +131,21 @@ __host__ __device__ constexpr ResidentLayout resident_layout_c(uint32_t l_max)
     off += 4ull * ly.hs;
     ly.off_HW = off;
     off += 4ull * ly.hs;
+    // The warps' union lists, in the seam tables' memory (reset after the
+    // unions) where that gives every warp at least 32 entries.
+    const uint32_t nwarps = (uint32_t)threads / 32u;
+    ly.off_LIST = ly.off_HK;
+    ly.seg = 4u * ly.hs / nwarps;
+    if (ly.seg < 32u) {
+        ly.off_LIST = off;
+        ly.seg = 32u;
+        off += 64ull * nwarps;
+    }
     ly.bytes = align16(off);
     return ly;
 }
 
-ResidentLayout resident_layout(uint32_t l_max, int threads)
-{
-    (void)threads;
-    return resident_layout_c(l_max);
-}
+ResidentLayout resident_layout(uint32_t l_max, int threads) { return resident_layout_c(l_max, threads); }
 
 int resident_max_l()
 {
@@ -163,7 +169,7 @@ int resident_default_threads(int l_max)
     if (l_max <= 32) return 32;
     if (l_max <= 64) return 128;
     if (l_max <= 96) return 256;
-    if (2 * (resident_layout_c((uint32_t)l_max).bytes + kStaticSmem) <= kSmemPerSm) return 512;
+    if (2 * (resident_layout_c((uint32_t)l_max, 512).bytes + kStaticSmem) <= kSmemPerSm) return 512;
     return 1024;
 }
 
@@ -193,6 +199,8 @@ struct Res {
     uint32_t *HK;  // seam hash keys: open root site, or kHashEmpty
     uint32_t *HW;  // seam union-find words (SeamWord)
     uint32_t hs, hs_log2;
+    unsigned short *LIST;  // union lists, `seg` entries per warp
+    uint32_t seg;
 };
 
 // walk_cap > 0 lowers the per-walk bound (and with it the per-thread loop
@@ -214,6 +222,7 @@ __device__ __forceinline__ Res make_res(unsigned char *smem, const ResidentLayou
     t.OV = (uint32_t *)(smem + ly.off_OV);
     t.FLIP = (uint32_t *)(smem + ly.off_FLIP);
     t.ROOT = (uint32_t *)(smem + ly.off_ROOT);
+    t.NEED = t.ROOT;  // read by the unions, before the roots are recorded
     t.RE = (const uint32_t *)(smem + ly.off_RE);
     t.SEAMV = (uint32_t *)(smem + ly.off_SEAMV);
     t.wrap = &red.wrap;
@@ -223,6 +232,8 @@ __device__ __forceinline__ Res make_res(unsigned char *smem, const ResidentLayou
     r.HW = (uint32_t *)(smem + ly.off_HW);
     r.hs = ly.hs;
     r.hs_log2 = 31u - __clz(ly.hs);
+    r.LIST = (unsigned short *)(smem + ly.off_LIST);
+    r.seg = ly.seg;
     return r;
 }
 
@@ -276,13 +287,13 @@ __device__ __forceinline__ void seam_union(const Res &r, uint32_t na, uint32_t n
     atomicOr(err, kErrUnionCap);
 }
 
-// Seam table reset (before the seam phase).
-__device__ __forceinline__ void seam_reset(const Res &r, uint32_t tid, uint32_t nthreads)
+// Seam table reset (before the seam phase): each warp resets the 1 / nwarps of
+// the two tables that its union list may have used, after its unions.
+__device__ __forceinline__ void seam_reset(const Res &r, uint32_t warp, uint32_t nwarps)
 {
-    for (uint32_t k = tid; k < r.hs; k += nthreads) {
-        r.HK[k] = kHashEmpty;
-        r.HW[k] = SeamWord::make(k, 0, 0);
-    }
+    const uint32_t per = 2u * r.hs / nwarps, end = (warp + 1u) * per;
+    for (uint32_t k = warp * per + (threadIdx.x & 31u); k < end; k += 32u)
+        r.HK[k] = k < r.hs ? kHashEmpty : SeamWord::make(k - r.hs, 0, 0);  // HW follows HK
 }
 
 // (b) Seam bonds: x seam (x = L-1 -> 0, crossing (1,0)) and y seam
@@ -334,20 +345,21 @@ __device__ __forceinline__ void phase_seam_propagate(const Res &r, uint32_t tid,
 // every site's word at its root; a sweep flips the clusters piece by piece
 // (flip_pieces), with the piece leaders' roots written when the
 // sweep is measured.
-template <int NT>
+template <int NT, bool kFew>
 __device__ __forceinline__ uint32_t resident_label(const Res &r, bool sweep, bool measure)
 {
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     constexpr uint32_t nwarps = NT / 32;
-    phase_heads<Word16>(r.t, warp, nwarps);
-    seam_reset(r, tid, NT);
-    for (uint32_t w = tid; w < r.t.g.NW; w += NT) r.t.ROOT[w] = 0u;
+    unsigned short *list = r.LIST + warp * r.seg;
+    phase_heads_open<kFew>(r.t, warp, nwarps);
     __syncthreads();
     RBIM_PHASE_MARK(1);
-    phase_union_open(r.t, tid, NT);
+    phase_union_open<kFew>(r.t, list, r.seg, warp, nwarps);
+    seam_reset(r, warp, nwarps);
     __syncthreads();
     RBIM_PHASE_MARK(2);
     phase_seam(r, tid, NT);
+    for (uint32_t w = tid; w < r.t.g.NW; w += NT) r.t.ROOT[w] = 0u;
     __syncthreads();
     RBIM_PHASE_MARK(3);
     phase_seam_propagate(r, tid, NT);
@@ -534,7 +546,7 @@ __device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, u
     __syncthreads();
 }
 
-// LC > 0: the launch's layout is resident_layout_c(LC), a compile-time
+// LC > 0: the launch's layout is resident_layout_c(LC, NT), a compile-time
 // constant; LC == 0: the layout passed in.
 template <int NT, int LC>
 __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
@@ -542,7 +554,7 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
                       long long *acc_i, double *acc_f, int32_t *records, int n_sweeps, int *queue, int *status,
                       ResidentLayout ly_arg)
 {
-    constexpr ResidentLayout kly = resident_layout_c(LC > 0 ? LC : 16);
+    constexpr ResidentLayout kly = resident_layout_c(LC > 0 ? LC : 16, NT);
     const ResidentLayout ly = LC > 0 ? kly : ly_arg;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Red<NT> red;
@@ -599,7 +611,7 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
             phase_activate<Word16>(t, make_rng(ch.key, sweep, ch.thr), warp, nwarps, tid, NT);
             __syncthreads();
             RBIM_PHASE_MARK(0);
-            const uint32_t nr = resident_label<NT>(res, true, measure);
+            const uint32_t nr = resident_label<NT, NT >= 512 && LC == 0>(res, true, measure);
             if (measure) {
                 long long rec[kRecLen];
                 const bool want_rec = records && ch.rec_off >= 0;
@@ -684,7 +696,7 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
         }
     }
     __syncthreads();
-    resident_label<NT>(res, false, false);
+    resident_label<NT, false>(res, false, false);
     // Exclusive prefix of root counts over words -> FLIP plane (rank base).
     const uint32_t per = (g.NW + NT - 1u) / NT;
     const uint32_t w0 = tid * per, w1 = min(g.NW, w0 + per);
@@ -724,7 +736,7 @@ cudaError_t launch_sweeps_lc(const rbim_chain_t *chains, int n_chains, int l_max
                              const uint32_t *coupling_pool, long long *acc_i, double *acc_f, int32_t *rec,
                              int n_sweeps, int grid, int *queue, int *status, cudaStream_t stream)
 {
-    const ResidentLayout ly = LC > 0 ? resident_layout_c(LC) : resident_layout(l_max, NT);
+    const ResidentLayout ly = LC > 0 ? resident_layout_c(LC, NT) : resident_layout(l_max, NT);
     cudaError_t e = cudaFuncSetAttribute(k_resident_sweeps<NT, LC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)ly.bytes);
     if (e != cudaSuccess) return e;
@@ -754,19 +766,24 @@ cudaError_t launch_sweeps_nt(const rbim_chain_t *chains, int n_chains, int l_max
                              const uint32_t *coupling_pool, long long *acc_i, double *acc_f, int32_t *rec,
                              int n_sweeps, int grid, int *queue, int *status, cudaStream_t stream)
 {
-    if (NT == 1024 && l_max > 128 && l_max <= 256)
-        return launch_sweeps_lc<NT, 256>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
-                                         n_sweeps, grid, queue, status, stream);
-    if (NT == 512 && l_max > 96 && l_max <= 128)
-        return launch_sweeps_lc<NT, 128>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
-                                         n_sweeps, grid, queue, status, stream);
-    if (NT == 512 && l_max > 128 && l_max <= 176 &&
-        2 * (resident_layout_c(176).bytes + kStaticSmem) <= kSmemPerSm)
-        return launch_sweeps_lc<NT, 176>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
-                                         n_sweeps, grid, queue, status, stream);
-    if (NT == 256 && l_max > 64 && l_max <= 96)
-        return launch_sweeps_lc<NT, 96>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
-                                        n_sweeps, grid, queue, status, stream);
+    if constexpr (NT == 1024) {
+        if (l_max > 128 && l_max <= 256)
+            return launch_sweeps_lc<NT, 256>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
+                                             n_sweeps, grid, queue, status, stream);
+    }
+    if constexpr (NT == 512) {
+        if (l_max > 96 && l_max <= 128)
+            return launch_sweeps_lc<NT, 128>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
+                                             n_sweeps, grid, queue, status, stream);
+        if (l_max > 128 && l_max <= 176 && 2 * (resident_layout_c(176, 512).bytes + kStaticSmem) <= kSmemPerSm)
+            return launch_sweeps_lc<NT, 176>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
+                                             n_sweeps, grid, queue, status, stream);
+    }
+    if constexpr (NT == 256) {
+        if (l_max > 64 && l_max <= 96)
+            return launch_sweeps_lc<NT, 96>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
+                                            n_sweeps, grid, queue, status, stream);
+    }
     return launch_sweeps_lc<NT, 0>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec, n_sweeps,
                                    grid, queue, status, stream);
 }
