@@ -56,17 +56,8 @@ __device__ __forceinline__ SweepRng make_rng(uint64_t key, uint64_t sweep, uint6
     return r;
 }
 
-// Occupation decision of one bond from its 16-bit draw u: u < thr_hi
-// accepts, u > thr_hi rejects, u == thr_hi (probability 2^-16) defers to the
-// low half v, drawn separately.  Returns 0 reject, 1 accept, 2 undecided.
-__device__ __forceinline__ uint32_t bond_decide(const SweepRng &rng, uint32_t u)
-{
-    if (rng.thr_all || u < rng.thr_hi) return 1u;
-    return u == rng.thr_hi ? 2u : 0u;
-}
-
-// Acceptance of one lane's Philox block of bond draws: bit s of the result
-// accepts the horizontal bond of word s (low half of word s of the block),
+// Acceptance of one lane's Philox block of bond draws, exact in every case:
+// bit s of the result accepts the horizontal bond of word s (low half of word s of the block),
 // bit 4 + s the vertical one (high half); satisfied masks are applied later.
 // A 16-bit draw equal to thr >> 16 defers to the low half drawn from stream
 // 3 (probability 2^-16 per bond), fetched when any lane of the warp needs it.
@@ -94,16 +85,122 @@ __device__ __forceinline__ uint32_t accept_block(const SweepRng &rng, const U4 &
     return acc;
 }
 
+// What every bond block of a sweep shares.  The counter of block b is {b,
+// sweep, 0}: in rounds 1 and 2 of Philox one of the two products has only
+// uniform factors, so the two rounds take one product each per block and the
+// rest folds into the constants below.  An accept of a 16-bit draw is one
+// compare against the threshold's high half, shifted to where the draw lies.
+struct BondDraw {
+    uint32_t k0, k1;          // round-3 keys
+    uint32_t u0, u1, u2, u3;  // uniform terms of rounds 1 (u0), 2 (u1, u2) and 3 (u3)
+    uint32_t top, both;       // thr >> 16 in the high half, and in both halves
+};
+
+__device__ __forceinline__ BondDraw make_bond_draw(const SweepRng &rng)
+{
+    const uint32_t k0 = (uint32_t)rng.key, k1 = (uint32_t)(rng.key >> 32), hi = (uint32_t)(rng.sweep >> 32);
+    BondDraw d;
+    const uint32_t c0 = __umulhi(kPhiloxM1, hi) ^ (uint32_t)rng.sweep ^ k0;  // word 0 after round 1
+    d.u0 = kStreamBond ^ k1;
+    d.u1 = kPhiloxM1 * hi ^ (k0 + kPhiloxW0);
+    d.u2 = __umulhi(kPhiloxM0, c0) ^ (k1 + kPhiloxW1);
+    d.k0 = k0 + 2u * kPhiloxW0;
+    d.k1 = k1 + 2u * kPhiloxW1;
+    d.u3 = kPhiloxM0 * c0 ^ d.k1;
+    d.top = rng.thr_hi << 16;
+    d.both = d.top | rng.thr_hi;
+    return d;
+}
+
+// philox_block(key, block, sweep, kStreamBond).
+__device__ __forceinline__ U4 bond_block(const BondDraw &d, uint32_t block)
+{
+    uint32_t c0, c1, c2, c3, k0 = d.k0, k1 = d.k1;
+    {
+        const uint32_t hi0 = __umulhi(kPhiloxM0, block), lo0 = kPhiloxM0 * block;
+        c2 = hi0 ^ d.u0;
+        const uint32_t hi1 = __umulhi(kPhiloxM1, c2), lo1 = kPhiloxM1 * c2;
+        c0 = hi1 ^ d.u1;
+        c1 = lo1;
+        c2 = lo0 ^ d.u2;
+    }
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+        const uint32_t hi0 = __umulhi(kPhiloxM0, c0), lo0 = kPhiloxM0 * c0;
+        const uint32_t hi1 = __umulhi(kPhiloxM1, c2), lo1 = kPhiloxM1 * c2;
+        c0 = hi1 ^ c1 ^ k0;
+        c2 = r == 2 ? hi0 ^ d.u3 : hi0 ^ c3 ^ k1;
+        c1 = lo1;
+        c3 = lo0;
+        k0 += kPhiloxW0;
+        k1 += kPhiloxW1;
+    }
+    return {c0, c1, c2, c3};
+}
+
+// The accepted bonds of one chunk of 128 sites as ballots: bit i of bh[s] and
+// bv[s] are the horizontal and vertical bond of the chunk's site 32 s + i,
+// drawn by lane i (r: its block).  A draw equal to thr >> 16 (a halfword of
+// `both` ^ word that is zero) is decided by its low half, for the whole chunk
+// in accept_block: 0.4 % of the chunks.
+__device__ __forceinline__ void accept_chunk(const SweepRng &rng, const BondDraw &d, const U4 &r, uint32_t block,
+                                             uint32_t bh[4], uint32_t bv[4])
+{
+    uint32_t eq = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const uint32_t w = u4_word(r, s), z = w ^ d.both;
+        eq |= (z - 0x00010001u) & ~z;
+        bh[s] = __ballot_sync(0xFFFFFFFFu, (w << 16) < d.top);
+        bv[s] = __ballot_sync(0xFFFFFFFFu, w < d.top);
+    }
+    if (__any_sync(0xFFFFFFFFu, (eq & 0x80008000u) != 0u)) {
+        const uint32_t acc = accept_block(rng, r, block);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            bh[s] = __ballot_sync(0xFFFFFFFFu, (acc >> s) & 1u);
+            bv[s] = __ballot_sync(0xFFFFFFFFu, (acc >> (4 + s)) & 1u);
+        }
+    }
+}
+
+// The draws of a group of up to eight chunks: lane j gets the accepted bonds
+// of the group's word j.  block0: this lane's block of the group's first
+// chunk.  Two chunks per iteration (a chunk past the group is drawn for
+// nothing): two independent Philox evaluations per lane.
+__device__ __forceinline__ void draw_group(const SweepRng &rng, const BondDraw &d, uint32_t block0, uint32_t nch,
+                                           uint32_t lane, uint32_t &oh, uint32_t &ov)
+{
+    oh = ov = 0xFFFFFFFFu;
+    if (rng.thr_all) return;
+    const uint32_t my_chunk = lane >> 2;
+    const bool s0 = lane & 1u, s1 = lane & 2u;
+    for (uint32_t k = 0; k < nch; k += 2u) {
+        const uint32_t block = block0 + 32u * k;
+        const U4 r0 = bond_block(d, block), r1 = bond_block(d, block + 32u);
+        uint32_t bh[4], bv[4];
+        accept_chunk(rng, d, r0, block, bh, bv);
+        if (my_chunk == k) {
+            oh = s1 ? (s0 ? bh[3] : bh[2]) : (s0 ? bh[1] : bh[0]);
+            ov = s1 ? (s0 ? bv[3] : bv[2]) : (s0 ? bv[1] : bv[0]);
+        }
+        accept_chunk(rng, d, r1, block + 32u, bh, bv);
+        if (my_chunk == k + 1u) {
+            oh = s1 ? (s0 ? bh[3] : bh[2]) : (s0 ? bh[1] : bh[0]);
+            ov = s1 ? (s0 ? bv[3] : bv[2]) : (s0 ? bv[1] : bv[0]);
+        }
+    }
+}
+
 // (a) Bond activation.  A 128-site chunk is four plane words; lane i of the
 // warp handling chunk c draws Philox block 32c + i, whose word s holds the
 // 16-bit draws of the horizontal (low half) and vertical (high half) bond of
 // site 128c + 32s + i, i.e. bit i of the chunk's word s, so that each ballot
 // is one word of the occupied-bond planes.  A warp takes a group of G
 // consecutive words (G = 32, eight chunks, while every warp still gets a
-// group): lane j first forms the satisfied masks of word j of the group --
-// every lane busy, coalesced loads -- then the warp draws the group's chunks
-// two at a time, and lane j keeps the ballots of its own word.  SEAMV must be
-// zero on entry.
+// group): lane j forms the satisfied masks of word j of the group -- every
+// lane busy, coalesced loads -- and keeps the ballots of its own word.  SEAMV
+// must be zero on entry.
 template <class WT>
 __device__ __forceinline__ void phase_activate_bonds(const Lat<WT> &t, const SweepRng &rng, uint32_t warp,
                                                      uint32_t nwarps)
@@ -115,49 +212,16 @@ __device__ __forceinline__ void phase_activate_bonds(const Lat<WT> &t, const Swe
     while (G > 4u && G * nwarps > g.NW) G >>= 1;
     const uint32_t ngroups = (g.NW + G - 1u) / G;
     const uint32_t nchunks = (g.NW + 3u) >> 2;
-    const uint32_t my_chunk = lane >> 2, my_s = lane & 3u;
+    const BondDraw draw = make_bond_draw(rng);
     for (uint32_t grp = warp; grp < ngroups; grp += nwarps) {
-        const uint32_t w = grp * G + lane;
-        const bool mine = lane < G && w < g.NW;
-        uint32_t sh = 0, sv = 0, re = 0;
-        if (mine) {
-            re = t.row_end(w);
-            const uint32_t v = g.valid(w);
-            const uint32_t s = S(w);
-            sh = ~(s ^ xnext_word(S, w, g) ^ t.JH[w]) & v;
-            sv = ~(s ^ ynext_word(S, w, g, re) ^ t.JV[w]) & v;
-        }
         const uint32_t c0 = grp * (G >> 2);
-        const uint32_t nch = min(G >> 2, nchunks - c0);
-        uint32_t oh = 0, ov = 0;
-        // Two chunks per iteration: two independent Philox evaluations per lane.
-        for (uint32_t k = 0; k < nch; k += 2u) {
-            const bool two = k + 1u < nch;
-            const U4 r0 = philox_block(rng.key, 32u * (c0 + k) + lane, rng.sweep, kStreamBond);
-            U4 r1{};
-            if (two) r1 = philox_block(rng.key, 32u * (c0 + k + 1u) + lane, rng.sweep, kStreamBond);
-            const uint32_t a0 = accept_block(rng, r0, 32u * (c0 + k) + lane);
-            const uint32_t a1 = two ? accept_block(rng, r1, 32u * (c0 + k + 1u) + lane) : 0u;
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const uint32_t bh0 = __ballot_sync(0xFFFFFFFFu, (a0 >> s) & 1u);
-                const uint32_t bv0 = __ballot_sync(0xFFFFFFFFu, (a0 >> (4 + s)) & 1u);
-                const uint32_t bh1 = __ballot_sync(0xFFFFFFFFu, (a1 >> s) & 1u);
-                const uint32_t bv1 = __ballot_sync(0xFFFFFFFFu, (a1 >> (4 + s)) & 1u);
-                if (my_s == (uint32_t)s) {
-                    if (my_chunk == k) {
-                        oh = bh0;
-                        ov = bv0;
-                    } else if (my_chunk == k + 1u) {
-                        oh = bh1;
-                        ov = bv1;
-                    }
-                }
-            }
-        }
-        if (mine) {
-            oh &= sh;
-            ov &= sv;
+        uint32_t oh, ov;
+        draw_group(rng, draw, 32u * c0 + lane, min(G >> 2, nchunks - c0), lane, oh, ov);
+        const uint32_t w = grp * G + lane;
+        if (lane < G && w < g.NW) {
+            const uint32_t re = t.row_end(w), v = g.valid(w), s = S(w);
+            oh &= ~(s ^ xnext_word(S, w, g) ^ t.JH[w]) & v;
+            ov &= ~(s ^ ynext_word(S, w, g, re) ^ t.JV[w]) & v;
             t.OH[w] = oh;
             t.OV[w] = ov & ~re;
             uint32_t seam = ov & re;

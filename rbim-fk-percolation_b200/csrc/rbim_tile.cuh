@@ -63,55 +63,20 @@ __device__ __forceinline__ void tile_activate(const Lat<Word16> &t, uint32_t *YS
     const uint32_t chunk0 = tl.b >> 7;
     const uint32_t last = tl.Tc - 1u;
     const bool end_is_row_end = ((tl.b + tl.Tc) % tl.L) == 0u;
-    // Groups of G consecutive words, as in phase_activate_bonds: lane j forms
-    // the satisfied masks of word j, then the warp draws the group's chunks
-    // two at a time and lane j keeps the ballots of its own word.
+    // Groups of G consecutive words, as in phase_activate_bonds.
     uint32_t G = 32u;
     while (G > 4u && G * nwarps > g.NW) G >>= 1;
     const uint32_t ngroups = (g.NW + G - 1u) / G;
-    const uint32_t my_chunk = lane >> 2, my_s = lane & 3u;
+    const BondDraw draw = make_bond_draw(rng);
     for (uint32_t grp = warp; grp < ngroups; grp += nwarps) {
-        const uint32_t w = grp * G + lane;
-        const bool mine = lane < G && w < g.NW;
-        uint32_t sh = 0, sv = 0, re = 0;
-        if (mine) {
-            const uint32_t v = g.valid(w);
-            re = tile_row_end(tl, w, v);
-            const uint32_t s = t.S[w];
-            sh = ~(s ^ extract_nowrap(t.S, (w << 5) + tl.L) ^ gJH[w]) & v;
-            sv = ~(s ^ tile_ynext(t.S, w, re, tl.L, front) ^ gJV[w]) & v;
-        }
         const uint32_t c0 = grp * (G >> 2);
-        const uint32_t nch = min(G >> 2, nchunks - c0);
-        uint32_t oh = 0, ov = 0;
-        for (uint32_t k = 0; k < nch; k += 2u) {
-            const bool two = k + 1u < nch;
-            const uint32_t b0 = 32u * (chunk0 + c0 + k) + lane, b1 = b0 + 32u;
-            const U4 r0 = philox_block(rng.key, b0, rng.sweep, kStreamBond);
-            U4 r1{};
-            if (two) r1 = philox_block(rng.key, b1, rng.sweep, kStreamBond);
-            const uint32_t a0 = accept_block(rng, r0, b0);
-            const uint32_t a1 = two ? accept_block(rng, r1, b1) : 0u;
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const uint32_t bh0 = __ballot_sync(0xFFFFFFFFu, (a0 >> s) & 1u);
-                const uint32_t bv0 = __ballot_sync(0xFFFFFFFFu, (a0 >> (4 + s)) & 1u);
-                const uint32_t bh1 = __ballot_sync(0xFFFFFFFFu, (a1 >> s) & 1u);
-                const uint32_t bv1 = __ballot_sync(0xFFFFFFFFu, (a1 >> (4 + s)) & 1u);
-                if (my_s == (uint32_t)s) {
-                    if (my_chunk == k) {
-                        oh = bh0;
-                        ov = bv0;
-                    } else if (my_chunk == k + 1u) {
-                        oh = bh1;
-                        ov = bv1;
-                    }
-                }
-            }
-        }
-        if (mine) {
-            oh &= sh;
-            ov &= sv;
+        uint32_t oh, ov;
+        draw_group(rng, draw, 32u * (chunk0 + c0) + lane, min(G >> 2, nchunks - c0), lane, oh, ov);
+        const uint32_t w = grp * G + lane;
+        if (lane < G && w < g.NW) {
+            const uint32_t v = g.valid(w), re = tile_row_end(tl, w, v), s = t.S[w];
+            oh &= ~(s ^ extract_nowrap(t.S, (w << 5) + tl.L) ^ gJH[w]) & v;
+            ov &= ~(s ^ tile_ynext(t.S, w, re, tl.L, front) ^ gJV[w]) & v;
             uint32_t keep = ov & ~re;
             if (w == (last >> 5) && !end_is_row_end) {
                 const uint32_t eb = 1u << (last & 31u);
