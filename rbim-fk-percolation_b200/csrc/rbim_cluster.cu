@@ -330,7 +330,7 @@ struct Dist {
 // dropped before they reach the cluster-wide union-find.
 template <int NT>
 __device__ __forceinline__ void tile_boundary(const Ctx &x, const Tile &tl, const Dist &d, uint32_t tile_end,
-                                              bool walk, uint32_t tid)
+                                              uint32_t tid)
 {
     const Lat<Word16> &t = x.t;
     const uint32_t rows_end = (tl.b + tl.Tc) / tl.L;  // rows x0 .. rows_end-1 end in the tile
@@ -384,13 +384,8 @@ __device__ __forceinline__ void tile_boundary(const Ctx &x, const Tile &tl, cons
         uint32_t ra = 0, rb = 0;
         if (live) {
             const unsigned short *ufb = tb == tl.c ? t.uf.w : d.cl.map_shared_rank(t.uf.w, tb);
-            if (walk) {
-                ra = tile_root_walk(t.uf.w, a, t.cap, d.err);
-                rb = (tb << 16) | tile_root_walk(ufb, bl, t.cap, d.err);
-            } else {
-                ra = tile_root(t.uf.w, a);
-                rb = (tb << 16) | tile_root(ufb, bl);
-            }
+            ra = tile_root_walk(t.uf.w, a, t.cap, d.err);
+            rb = (tb << 16) | tile_root_walk(ufb, bl, t.cap, d.err);
         }
         // A bond joining the same two tile roots with the same seam crossing
         // as the previous lane's closes a loop of winding zero (paths inside a
@@ -453,22 +448,15 @@ __device__ __forceinline__ uint32_t node_root(const Ctx &x, uint32_t k)
 // half carries its root node between the two halves of the propagation).
 __device__ __forceinline__ uint32_t node_key(uint32_t hk) { return hk & 0xFFFFu; }
 
-// The open-tile union and root walks as separate (non-inlined) functions: the
-// cluster kernel keeps more state live across its phases than the resident
-// one, and compiled inline these pointer-chasing loops lose registers to it.
+// The open-tile unions as a separate (non-inlined) function: the cluster
+// kernel keeps more state live across its phases than the resident one, and
+// compiled inline this pointer-chasing loop loses registers to it.
 template <int NT>
 static __device__ __noinline__ void cluster_union(const Lat<Word16> &t, unsigned short *list, uint32_t seg,
                                                   uint32_t warp)
 {
     phase_union_open<false>(t, list, seg, warp, NT / 32);
 }
-
-template <int NT>
-static __device__ __noinline__ void cluster_roots(const Lat<Word16> &t, uint32_t tid)
-{
-    (void)phase_roots_flat(t, tid, NT);
-}
-
 
 // NT threads per CTA.  LC > 0: the layout is cluster_layout_c(LC, CC), a
 // compile-time constant, and the cluster has CC CTAs; LC == 0: the layout
@@ -561,19 +549,11 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             for (uint32_t k = warp * share + lane; k < (warp + 1u) * share; k += 32u)
                 x.HW[k] = Word64::make((c << 16) | k, 0, 0);
             __syncthreads();
-            // With at least one word per thread the roots are found in one
-            // pass with the flip, after the boundary stage (roots_flip_pieces);
-            // the boundary bonds' tile roots are then found by read-only walks.
-            const bool merged = t.g.NW >= (uint32_t)NT;
-            if (!merged) {
-                for (uint32_t w = tid; w < t.g.NW; w += NT) t.ROOT[w] = 0u;
-                __syncthreads();
-                cluster_roots<NT>(t, tid);
-                __syncthreads();
-            }
-            cl.sync();  // every tile's unions (and roots) are final
+            cl.sync();  // every tile's unions are final
 
-            tile_boundary<NT>(x, tl, d, red.tile_end, merged, tid);
+            // The roots are found in one pass with the flip, after the
+            // boundary stage, which finds its tile roots by read-only walks.
+            tile_boundary<NT>(x, tl, d, red.tile_end, tid);
             cl.sync();  // every boundary union is done
 
             // Root node of each of this tile's nodes, kept in the high half of
@@ -604,14 +584,11 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                 }
             }
             __syncthreads();
-            // Flip run pieces by their tile root's FLIP bit; every piece
-            // leader's word is left holding its tile root (without the merged
-            // pass only in measured sweeps), and the merged pass also sets the
-            // ROOT bits.
-            if (merged)
-                (void)roots_flip_pieces(t, tid, NT);
-            else
-                flip_pieces(t, tid, NT, measure);
+            // Tile roots, ROOT bits and flip; in measured sweeps the sites of
+            // the tile cluster most likely to be its largest go to the OH
+            // plane, which is free until the next activation.
+            const uint32_t likely = measure ? likely_largest(t) : 0u;
+            roots_flip_sites<true, 4>(t, measure ? t.OH : nullptr, likely, warp, nwarps);
             __syncthreads();
             cl.sync();  // every flip is done
             tile_halo<NT>(x, tl, cl, red, tid);
@@ -627,7 +604,20 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             // (a root points at itself): afterwards the word of root m reads
             // m + size - 1, below 65536 because m is the smallest site of its tile
             // cluster, so no add carries out of its 16 bits (tile_size decodes it).
-            count_pieces<true>(t, u16, warp, nwarps);
+            // The likely largest tile cluster is counted, and its magnetization
+            // summed, by popcounts.
+            count_pieces<true>(t, u16, t.OH, warp, nwarps);
+            int likely_m = 0;
+            {
+                uint32_t in = 0;
+                for (uint32_t w = tid; w < t.g.NW; w += NT) {
+                    const uint32_t m = t.OH[w];
+                    in += __popc(m) - (w == likely >> 5 ? 1u : 0u);
+                    likely_m += (int)__popc(m) - 2 * (int)__popc(m & t.S[w]);
+                }
+                in = __reduce_add_sync(0xFFFFFFFFu, in);
+                if (lane == 0 && in) add16(u16, likely, in);
+            }
             __syncthreads();
             // FLIP (no longer needed this sweep) becomes the plane of node
             // marks; OV still gives the run pieces of the |M_C| pass.
@@ -748,17 +738,18 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             // do not use it).
             const bool second = records && ch.rec_off >= 0;
             if (many) {
-                // Tile roots of the largest cluster, marked in OH, and with
-                // `second` those of the second largest in FLIP (whose node
-                // marks are no longer needed).
+                // Tile roots of the largest cluster, marked in FLIP (whose
+                // node marks are no longer needed); with `second` in OH, and
+                // those of the second largest in FLIP.
+                uint32_t *mark = second ? t.OH : t.FLIP;
                 for (uint32_t w = tid; w < t.g.NW; w += NT) {
-                    t.OH[w] = 0u;
-                    if (second) t.FLIP[w] = 0u;
+                    t.FLIP[w] = 0u;
+                    if (second) t.OH[w] = 0u;
                 }
                 __syncthreads();
                 if (tid == 0 && g1 >= tl.b && g1 < tl.b + tl.Tc) {
                     const uint32_t m = g1 - tl.b;
-                    atomicOr(t.OH + (m >> 5), 1u << (m & 31u));
+                    atomicOr(mark + (m >> 5), 1u << (m & 31u));
                 }
                 if (second && tid == 0 && g2 >= tl.b && g2 < tl.b + tl.Tc) {
                     const uint32_t m = g2 - tl.b;
@@ -771,7 +762,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                     const uint32_t gr = rt * tl.T + *cl.map_shared_rank(x.HK + (r & 0xFFFFu), rt);
                     if (gr == g1) {
                         const uint32_t m = x.HK[k];
-                        atomicOr(t.OH + (m >> 5), 1u << (m & 31u));
+                        atomicOr(mark + (m >> 5), 1u << (m & 31u));
                     } else if (second && gr == g2) {
                         const uint32_t m = x.HK[k];
                         atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
@@ -779,22 +770,25 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                 }
                 __syncthreads();
                 int mc = 0, mc2 = 0;
-                // One lane per word, one test per run piece: a piece leader's
-                // word holds its tile root (the root's own word its size).
+                if (!second && ((mark[likely >> 5] >> (likely & 31u)) & 1u)) mc = likely_m;
+                // One lane per word, one test per run piece, from the top: a
+                // piece leader's word holds its tile root (the root's own word
+                // its size).  Pieces of the likely largest are summed above.
                 for (uint32_t w = tid; w < t.g.NW; w += NT) {
-                    const uint32_t valid = t.g.valid(w);
-                    uint32_t lead = piece_leaders(t, w, valid);
+                    const uint32_t valid = t.g.valid(w), skip = second ? 0u : t.OH[w];
                     const uint32_t roots = t.ROOT[w], sw = t.S[w];
-                    const uint32_t nv = (uint32_t)__popc(valid);
-                    while (lead) {
-                        const uint32_t b = __ffs(lead) - 1u;
-                        lead &= lead - 1u;
-                        const uint32_t end = lead ? (uint32_t)(__ffs(lead) - 1) : nv;
+                    uint32_t cut = piece_leaders(t, w, valid) & ~(skip & ((skip << 1) | 1u));
+                    uint32_t left = valid;  // the bits below the last piece
+                    while (cut) {
+                        const uint32_t b = 31u - __clz(cut), bit = 1u << b;
+                        const uint32_t pm = left & (0u - bit);
+                        cut ^= bit;
+                        left ^= pm;
+                        if (skip & bit) continue;
                         const uint32_t n = (w << 5) + b;
-                        const uint32_t r = ((roots >> b) & 1u) ? n : (uint32_t)u16[n];
-                        const uint32_t pm = (end - b == 32u) ? 0xFFFFFFFFu : (((1u << (end - b)) - 1u) << b);
+                        const uint32_t r = roots & bit ? n : (uint32_t)u16[n];
                         const int m = (int)__popc(pm) - 2 * (int)__popc(pm & sw);
-                        if ((t.OH[r >> 5] >> (r & 31u)) & 1u) mc += m;
+                        if ((mark[r >> 5] >> (r & 31u)) & 1u) mc += m;
                         if (second && ((t.FLIP[r >> 5] >> (r & 31u)) & 1u)) mc2 += m;
                     }
                 }

@@ -572,20 +572,14 @@ __device__ __forceinline__ void grid_boundary(const GTile &x, const Tile &tl, co
 }
 
 
-// The open-tile union and root walks as separate (non-inlined) functions, as
-// in the cluster engine: inline, these pointer-chasing loops lose registers
-// to the state the kernel keeps live across its phases.
+// The open-tile unions as a separate (non-inlined) function, as in the cluster
+// engine: inline, this pointer-chasing loop loses registers to the state the
+// kernel keeps live across its phases.
 template <int NT>
 static __device__ __noinline__ void grid_union(const Lat<Word16> &t, unsigned short *list, uint32_t seg,
                                                uint32_t warp)
 {
     phase_union_open<true>(t, list, seg, warp, NT / 32);
-}
-
-template <int NT>
-static __device__ __noinline__ void grid_roots(const Lat<Word16> &t, uint32_t tid)
-{
-    (void)phase_roots_flat(t, tid, NT);
 }
 
 struct GridArgs {
@@ -745,14 +739,17 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
         RBIM_GRID_MARK(0);
         for (uint32_t w = tid; w < t.g.NW; w += NT) ws.FLIPG[(tl.b >> 5) + w] = t.FLIP[w];
         phase_heads_open<true>(t, warp, nwarps);
-        for (uint32_t w = tid; w < t.g.NW; w += NT) t.ROOT[w] = 0u;
         __syncthreads();
         RBIM_GRID_MARK(1);
         const uint32_t seg = ly.list / nwarps;  // union lists, in the node lists' memory
         grid_union<NT>(t, (unsigned short *)x.NK + warp * seg, seg, warp);
         __syncthreads();
         RBIM_GRID_MARK(2);
-        grid_roots<NT>(t, tid);
+        // Every site's word at its tile root, and the ROOT plane.
+        if (t.g.NW <= nwarps)
+            roots_flip_sites<false, 1>(t, nullptr, 0u, warp, nwarps);
+        else
+            roots_flip_sites<false, 4>(t, nullptr, 0u, warp, nwarps);
         for (uint32_t w = tid; w < t.g.NW; w += NT) x.NODE[w] = 0u;
         __syncthreads();
         RBIM_GRID_MARK(3);
@@ -784,28 +781,30 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
             }
         }
         __syncthreads();
-        // Flip by the tile root's FLIP bit: run piece by run piece (a
-        // measured sweep also leaves every piece leader's word holding its
-        // tile root), or, in tiles with fewer than a quarter as many words as
-        // threads, site by site (every site's word then holds its tile root).
         RBIM_GRID_MARK(8);
-        const bool per_site = 4u * t.g.NW <= NT;
-        if (!per_site)
-            flip_pieces(t, tid, NT, measure);
-        else
-            phase_sites<Word16>(t, warp, nwarps, true, false);
-        __syncthreads();
+        // Flip by the tile root's FLIP bit, one lane per site, and write the
+        // spins back.
+        for (uint32_t w = warp; w < t.g.NW; w += nwarps) {
+            const uint32_t n = (w << 5) + lane;
+            const uint32_t r = t.uf.ld(n < tl.Tc ? n : 0u);
+            const uint32_t f = __ballot_sync(0xFFFFFFFFu, n < tl.Tc && ((t.FLIP[r >> 5] >> (r & 31u)) & 1u));
+            if (lane == 0) {
+                const uint32_t s = t.S[w] ^ f;
+                t.S[w] = s;
+                gS[w] = s & t.g.valid(w);
+            }
+        }
         RBIM_GRID_MARK(9);
-        for (uint32_t w = tid; w < tl.tw; w += NT) gS[w] = t.S[w] & t.g.valid(w);
         // Measured sweeps: cluster sizes before the barrier that publishes the
         // spins, so that one barrier also completes the merged sizes.
         uint32_t nloc = 0;
         if (measure) {
+            __syncthreads();  // the flips have read the roots
             // Tile cluster sizes minus one added onto each tile root's own index
             // (a root points at itself): afterwards the word of root m reads
             // m + size - 1, below 65536 because m is the smallest site of its tile
             // cluster, so no add carries out of its 16 bits (tile_size decodes it).
-            count_pieces<true>(t, u16, warp, nwarps);
+            count_pieces<true>(t, u16, nullptr, warp, nwarps);
             __syncthreads();
             RBIM_GRID_MARK(12);
             // Node sizes into the root nodes' words (the high half of a root's
@@ -958,35 +957,15 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
                     atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
             }
             __syncthreads();
-            // One lane per word, one test per run piece: a piece leader's
-            // word holds its tile root; site by site (one warp per word)
-            // where the flip went site by site.
-            if (per_site) {
-                for (uint32_t w = warp; w < t.g.NW; w += nwarps) {
-                    const uint32_t n = (w << 5) + lane;
-                    if (n >= tl.Tc) continue;
-                    const uint32_t r = ((t.ROOT[w] >> lane) & 1u) ? n : (uint32_t)u16[n];
-                    const int m = 1 - 2 * (int)((t.S[w] >> lane) & 1u);
-                    if ((t.OH[r >> 5] >> (r & 31u)) & 1u) mc += m;
-                    if (second && ((t.FLIP[r >> 5] >> (r & 31u)) & 1u)) mc2 += m;
-                }
-            }
-            for (uint32_t w = tid; w < t.g.NW && !per_site; w += NT) {
-                const uint32_t valid = t.g.valid(w);
-                uint32_t lead = piece_leaders(t, w, valid);
-                const uint32_t roots = t.ROOT[w], sw = t.S[w];
-                const uint32_t nv = (uint32_t)__popc(valid);
-                while (lead) {
-                    const uint32_t b = __ffs(lead) - 1u;
-                    lead &= lead - 1u;
-                    const uint32_t end = lead ? (uint32_t)(__ffs(lead) - 1) : nv;
-                    const uint32_t n = (w << 5) + b;
-                    const uint32_t r = ((roots >> b) & 1u) ? n : (uint32_t)u16[n];
-                    const uint32_t pm = (end - b == 32u) ? 0xFFFFFFFFu : (((1u << (end - b)) - 1u) << b);
-                    const int m = (int)__popc(pm) - 2 * (int)__popc(pm & sw);
-                    if ((t.OH[r >> 5] >> (r & 31u)) & 1u) mc += m;
-                    if (second && ((t.FLIP[r >> 5] >> (r & 31u)) & 1u)) mc2 += m;
-                }
+            // One lane per site: a site's word holds its tile root (a root's
+            // own word its size).
+            for (uint32_t w = warp; w < t.g.NW; w += nwarps) {
+                const uint32_t n = (w << 5) + lane;
+                if (n >= tl.Tc) continue;
+                const uint32_t r = ((t.ROOT[w] >> lane) & 1u) ? n : (uint32_t)u16[n];
+                const int m = 1 - 2 * (int)((t.S[w] >> lane) & 1u);
+                if ((t.OH[r >> 5] >> (r & 31u)) & 1u) mc += m;
+                if (second && ((t.FLIP[r >> 5] >> (r & 31u)) & 1u)) mc2 += m;
             }
         }
         for (int o = 16; o > 0; o >>= 1) {

@@ -369,78 +369,6 @@ __device__ __forceinline__ void phase_union_open(const Lat<Word16> &t, unsigned 
 #endif
 }
 
-// (c) Roots of the run heads (see phase_roots), as a flat per-thread loop
-// over the heads of the thread's slices: read-only walks, each head's final
-// root written by the head's own thread.  ROOT must be zero on entry.
-// Returns the number of roots this thread found.
-// Next head of the thread's slices into (h, x), or false when there is none.
-__device__ __forceinline__ bool next_head(const Lat<Word16> &t, const Slices &sl, uint32_t nthreads, uint32_t &item,
-                                          uint32_t &pending, uint32_t &base, uint32_t &h)
-{
-    while (!pending && item < sl.items) {
-        const uint32_t w = sl.word(item);
-        pending = head_mask(t.OV, w, t.g.valid(w)) & sl.mask(item);
-        base = w << 5;
-        item += nthreads;
-    }
-    if (!pending) return false;
-    h = base + (uint32_t)(__ffs(pending) - 1);
-    pending &= pending - 1u;
-    return true;
-}
-
-__device__ __forceinline__ uint32_t phase_roots_flat(const Lat<Word16> &t, uint32_t tid, uint32_t nthreads)
-{
-    const Geom &g = t.g;
-    const Slices sl = make_slices(g.NW, nthreads);
-    uint32_t item = tid, pending = 0, base = 0, nroots = 0;
-    // Two walks in flight per thread: heads h0, h1 at positions x0, x1.
-    uint32_t h0 = 0, h1 = 0, x0 = 0, x1 = 0;
-    bool a0 = next_head(t, sl, nthreads, item, pending, base, h0);
-    bool a1 = a0 && next_head(t, sl, nthreads, item, pending, base, h1);
-    x0 = h0;
-    x1 = h1;
-    const uint32_t cap = 64u * t.cap;  // 64 walks of t.cap steps (64 N + 4096 by default)
-    for (uint32_t it = 0; a0 || a1; ++it) {
-        if (it >= cap) {
-            atomicOr(t.err, kErrFindCap);
-            break;
-        }
-        const uint32_t p0 = t.uf.ld(x0), p1 = t.uf.ld(x1);
-        const bool r0 = a0 && p0 == x0, r1 = a1 && p1 == x1;
-        x0 = p0;
-        x1 = p1;
-        if (r0) {
-            if (x0 != h0) {
-                t.uf.st(h0, (unsigned short)x0);
-            } else {
-                atomicOr(t.ROOT + (h0 >> 5), 1u << (h0 & 31u));
-                ++nroots;
-            }
-            a0 = next_head(t, sl, nthreads, item, pending, base, h0);
-            x0 = h0;
-        }
-        if (r1) {
-            if (x1 != h1) {
-                t.uf.st(h1, (unsigned short)x1);
-            } else {
-                atomicOr(t.ROOT + (h1 >> 5), 1u << (h1 & 31u));
-                ++nroots;
-            }
-            a1 = next_head(t, sl, nthreads, item, pending, base, h1);
-            x1 = h1;
-        }
-    }
-    return nroots;
-}
-
-__device__ __forceinline__ uint32_t warp_sum(uint32_t v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
-
 // Run pieces: the sites of a word split into maximal runs of occupied
 // y-bonds; every piece starts at a run head or at bit 0 of the word and all
 // its sites share one root.  Bits of the pieces' first sites.
@@ -456,57 +384,49 @@ __device__ __forceinline__ void add16(unsigned short *base, uint32_t i, uint32_t
     atomicAdd((unsigned int *)(base + (i & ~1u)), v << (16u * (i & 1u)));
 }
 
-// Cluster sizes into the root words (after the sites pass, every non-root
-// site's word holds its root): one add per run piece, the sites of a word
-// split into maximal runs sharing a root.  With at least 32 words per warp,
-// each lane takes a word of its warp's block of 32 and walks the word's
-// pieces, summing consecutive pieces of one root in a register; at the end
-// of the block the lanes holding the same root add their sums in one atomic,
-// so a giant cluster sees one add per block instead of one per piece.
+// Cluster sizes into the root words (every piece leader's word holds its
+// root): one add per run piece, the sites of a word split into maximal runs
+// sharing a root.  With at least 32 words per warp each lane takes a word and
+// walks its pieces from the top, so that a piece ends where the last one
+// began; with fewer the lanes are the sites of a word.
+// skip (or null): plane of the sites of one cluster, counted by popcounts
+// elsewhere; without it the largest cluster's root would take most of the
+// adds, one after the other.
 // kMinusOne: the piece that starts at the root adds one less, so that a root
 // word holds size - 1 (a tile of 65536 sites then still fits 16 bits).
 // Each root word must hold zero or the root's own index on entry (a root
 // points at itself, so counting onto it needs no zeroing pass; the caller
 // then subtracts the index).
 template <bool kMinusOne>
-__device__ __forceinline__ void count_pieces(const Lat<Word16> &t, unsigned short *u16, uint32_t warp,
-                                             uint32_t nwarps)
+__device__ __forceinline__ void count_pieces(const Lat<Word16> &t, unsigned short *u16, const uint32_t *skip,
+                                             uint32_t warp, uint32_t nwarps)
 {
     const Geom &g = t.g;
     const uint32_t lane = threadIdx.x & 31u;
     if (g.NW >= 32u * nwarps) {
-        for (uint32_t w0 = warp << 5; w0 < g.NW; w0 += nwarps << 5) {
-            const uint32_t w = w0 + lane;
-            uint32_t acc_r = 0xFFFFFFFFu, acc = 0;
-            if (w < g.NW) {
-                const uint32_t valid = g.valid(w);
-                uint32_t lead = piece_leaders(t, w, valid);
-                const uint32_t roots = t.ROOT[w];
-                const uint32_t nv = (uint32_t)__popc(valid);
-                while (lead) {
-                    const uint32_t b = __ffs(lead) - 1u;
-                    lead &= lead - 1u;
-                    const uint32_t end = lead ? (uint32_t)(__ffs(lead) - 1) : nv;
+        for (uint32_t w = (warp << 5) + lane; w < g.NW; w += nwarps << 5) {
+            const uint32_t valid = g.valid(w), roots = t.ROOT[w], sk = skip ? skip[w] : 0u;
+            // Where counted pieces begin or end: not between two skipped ones.
+            uint32_t cut = piece_leaders(t, w, valid) & ~(sk & ((sk << 1) | 1u));
+            uint32_t end = 32u - __clz(valid);
+            while (cut) {
+                const uint32_t b = 31u - __clz(cut), bit = 1u << b;
+                cut ^= bit;
+                if (!(sk & bit)) {
                     const uint32_t n = (w << 5) + b;
-                    const bool is_root = (roots >> b) & 1u;
+                    const bool is_root = roots & bit;
                     const uint32_t r = is_root ? n : (uint32_t)u16[n];
-                    if (r != acc_r) {
-                        if (acc) add16(u16, acc_r, acc);
-                        acc_r = r;
-                        acc = 0;
-                    }
-                    acc += end - b - ((kMinusOne && is_root) ? 1u : 0u);
+                    add16(u16, r, end - b - ((kMinusOne && is_root) ? 1u : 0u));
                 }
+                end = b;
             }
-            const uint32_t grp = __match_any_sync(0xFFFFFFFFu, acc_r);
-            const uint32_t sum = __reduce_add_sync(grp, acc);
-            if (acc_r != 0xFFFFFFFFu && lane == (uint32_t)(__ffs(grp) - 1) && sum) add16(u16, acc_r, sum);
         }
     } else {
         for (uint32_t w = warp; w < g.NW; w += nwarps) {
             const uint32_t valid = g.valid(w);
             const uint32_t lead = piece_leaders(t, w, valid);
-            if ((lead >> lane) & 1u) {
+            const uint32_t todo = skip ? lead & ~skip[w] : lead;
+            if ((todo >> lane) & 1u) {
                 const uint32_t n = (w << 5) + lane;
                 const uint32_t next = lead & ~mask_le(lane);
                 const uint32_t end = next ? (uint32_t)(__ffs(next) - 1) : (uint32_t)__popc(valid);
@@ -518,93 +438,80 @@ __device__ __forceinline__ void count_pieces(const Lat<Word16> &t, unsigned shor
     }
 }
 
-// Root of any site n once the roots pass is done: every parent is a run head
-// (heads are the initial parents, roots are heads, and hooks, path halving
-// and the seam merge only ever point at roots or grandparents) and every head
-// then points at its root (a root at itself), so two loads reach it.
-__device__ __forceinline__ uint32_t piece_root(const unsigned short *u16, uint32_t n) { return u16[u16[n]]; }
-
-// The cluster flip of a sweep, one lane per word and one root lookup per run
-// piece instead of per site: the sites of a word split into pieces (maximal
-// runs of occupied y-bonds cut at the word boundary) that share a root, and a
-// piece flips as a whole when its root's FLIP bit is set.  With
-// `leader_roots` the leader of every piece that does not head its run (bit 0
-// of a word inside a run) also gets its root written, so that afterwards the
-// word of every piece leader holds its root, which the cluster-size count and
-// the |M_C| pass read.  Non-head words are nobody's parent, so the writes do
-// not disturb the lookups of other lanes.
-__device__ __forceinline__ void flip_pieces(const Lat<Word16> &t, uint32_t tid, uint32_t nthreads,
-                                                     bool leader_roots)
+// The root most likely to have the largest cluster: of 32 sites spread over
+// the lattice, the root that most of them share (the smallest such root).
+// Every warp finds the same one, by read-only walks.
+__device__ __forceinline__ uint32_t likely_largest(const Lat<Word16> &t)
 {
-    const Geom &g = t.g;
-    unsigned short *u16 = t.uf.w;
-    for (uint32_t w = tid; w < g.NW; w += nthreads) {
-        const uint32_t valid = g.valid(w);
-        const uint32_t heads = head_mask(t.OV, w, valid);
-        uint32_t lead = (heads | 1u) & valid;
-        const uint32_t nv = (uint32_t)__popc(valid);
-        uint32_t fl = 0;
-        while (lead) {
-            const uint32_t b = __ffs(lead) - 1u;
-            lead &= lead - 1u;
-            const uint32_t end = lead ? (uint32_t)(__ffs(lead) - 1) : nv;
-            const uint32_t n = (w << 5) + b;
-            const uint32_t r = piece_root(u16, n);
-            if ((t.FLIP[r >> 5] >> (r & 31u)) & 1u) fl |= (end - b == 32u) ? 0xFFFFFFFFu : (((1u << (end - b)) - 1u) << b);
-            if (leader_roots && !((heads >> b) & 1u)) u16[n] = (unsigned short)r;
-        }
-        if (fl) t.S[w] ^= fl;
-    }
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t r = uf_root_ro<Word16>(t.uf, (uint32_t)(((2u * lane + 1u) * t.g.N) >> 6), t.cap, t.err);
+    const uint32_t same = __popc(__match_any_sync(0xFFFFFFFFu, r));
+    return 0xFFFFu - (__reduce_max_sync(0xFFFFFFFFu, (same << 16) | (0xFFFFu - r)) & 0xFFFFu);
 }
 
-// Roots and cluster flip of a sweep in one pass, one lane per word and one
-// walk per run piece (the sites of a word split into pieces -- maximal runs
-// of occupied y-bonds cut at the word boundary -- that share a root).  A
-// piece's leader walks read-only up to its root; the root is then written
-// into the leader's word (for a run head this is the final compression the
-// separate roots pass would make, and the count and |M_C| passes read it
-// for every leader), the piece flips as a whole with its root's FLIP bit,
-// and a leader that is its own root sets its ROOT bit.  Walks of other lanes
-// running at the same time may read a head's old parent or its final root;
-// both are ancestors, so every walk ends at the right root.  Roots' words are
-// never written.  Returns the number of roots this thread found.
-__device__ __forceinline__ uint32_t roots_flip_pieces(const Lat<Word16> &t, uint32_t tid, uint32_t nthreads)
+// Roots and cluster flip in one pass, one lane per site and K consecutive
+// words at a time (K independent chains of loads): all lanes walk up to their
+// roots together (a word's walks end within a step or two of each other, and
+// the sites of a run or of one cluster load the same words), the site's word
+// gets its root, and ballots give the word's ROOT bits, its flips (kFlip) and,
+// with `in`, its sites in the cluster rooted at `root`.  Walks of other warps
+// running at the same time may read a site's old parent or its root; both are
+// ancestors, and roots' words never change.
+//
+// Bound by the latency and bank conflicts of the gathers.  Every lane works
+// (one lane per word with a walk per run piece left half of them idle: 64 k
+// cycles per L = 256 sweep on one SM, 39 k this way), and leaving out the loads
+// of lanes that have arrived costs more in branches than it saves (71 k).
+template <bool kFlip, int K>
+__device__ __forceinline__ void roots_flip_sites(const Lat<Word16> &t, uint32_t *in, uint32_t root, uint32_t warp,
+                                                 uint32_t nwarps)
 {
+    const uint32_t lane = threadIdx.x & 31u;
     const Geom &g = t.g;
     const UF<Word16> &uf = t.uf;
-    uint32_t nroots = 0;
-    for (uint32_t w = tid; w < g.NW; w += nthreads) {
-        const uint32_t valid = g.valid(w);
-        uint32_t lead = (head_mask(t.OV, w, valid) | 1u) & valid;
-        const uint32_t nv = (uint32_t)__popc(valid);
-        uint32_t fl = 0, rootbits = 0;
-        while (lead) {
-            const uint32_t b = __ffs(lead) - 1u;
-            lead &= lead - 1u;
-            const uint32_t end = lead ? (uint32_t)(__ffs(lead) - 1) : nv;
-            const uint32_t n = (w << 5) + b;
-            uint32_t x = uf.ld(n);
-            for (uint32_t it = 0;; ++it) {
-                const uint32_t p = uf.ld(x);
-                if (p == x) break;
-                if (it >= t.cap) {
-                    atomicOr(t.err, kErrFindCap);
-                    break;
-                }
-                x = p;
+    for (uint32_t w0 = K * warp; w0 < g.NW; w0 += K * nwarps) {
+        const uint32_t n0 = (w0 << 5) + lane;
+        // Lanes past the lattice walk from site 0, which is a root.  Two steps
+        // a vote.
+        uint32_t r[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) r[k] = uf.ld(n0 + 32u * k < g.N ? n0 + 32u * k : 0u);
+        for (uint32_t it = 0;; ++it) {
+            uint32_t p[K];
+            bool moved = false;
+#pragma unroll
+            for (int k = 0; k < K; ++k) p[k] = uf.ld(r[k]);
+#pragma unroll
+            for (int k = 0; k < K; ++k) r[k] = uf.ld(p[k]);
+#pragma unroll
+            for (int k = 0; k < K; ++k) moved |= p[k] != r[k];
+            if (!__any_sync(0xFFFFFFFFu, moved)) break;
+            if (it >= t.cap) {
+                if (moved) atomicOr(t.err, kErrFindCap);
+                break;
             }
-            if (x == n) {
-                rootbits |= 1u << b;
-                ++nroots;
-            } else {
-                uf.st(n, (unsigned short)x);
-            }
-            if ((t.FLIP[x >> 5] >> (x & 31u)) & 1u) fl |= (end - b == 32u) ? 0xFFFFFFFFu : (((1u << (end - b)) - 1u) << b);
         }
-        t.ROOT[w] = rootbits;
-        if (fl) t.S[w] ^= fl;
+        uint32_t roots = 0, flips = 0, members = 0;  // lane k: of word w0 + k
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t n = n0 + 32u * k;
+            const bool ok = n < g.N;
+            if (ok) uf.st(n, (unsigned short)r[k]);
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, ok && r[k] == n);
+            const uint32_t f = kFlip ? __ballot_sync(0xFFFFFFFFu, ok && ((t.FLIP[r[k] >> 5] >> (r[k] & 31u)) & 1u)) : 0u;
+            const uint32_t c = __ballot_sync(0xFFFFFFFFu, ok && r[k] == root);
+            if (lane == k) {
+                roots = b;
+                flips = f;
+                members = c;
+            }
+        }
+        if (lane < K && w0 + lane < g.NW) {
+            t.ROOT[w0 + lane] = roots;
+            if (kFlip) t.S[w0 + lane] ^= flips;
+            if (in) in[w0 + lane] = members;
+        }
     }
-    return nroots;
 }
 
 }  // namespace rbim

@@ -177,10 +177,9 @@ int resident_default_threads(int l_max)
 template <int NT>
 struct Red {
     uint32_t k1[NT / 32], k2[NT / 32];
-    uint32_t unsat[NT / 32], downs[NT / 32], roots[NT / 32];
+    uint32_t unsat[NT / 32], downs[NT / 32], roots[NT / 32], in[NT / 32], in_downs[NT / 32];
     int mc[NT / 32], mc2[NT / 32];
     int item, wrap, err;
-    uint32_t g1, g2, s1, s2;
     // State of the chain being processed; only thread 0 updates it.
     Acc acc;
     long long cur_bin;
@@ -340,16 +339,20 @@ __device__ __forceinline__ void phase_seam_propagate(const Res &r, uint32_t tid,
 }
 
 // The labelling stages shared by the sweep and label kernels, from occupied
-// bond planes to final roots; barriers between stages.  Returns the number of
-// roots counted by this warp.  The label kernel (sweep = false) then points
-// every site's word at its root; a sweep flips the clusters piece by piece
-// (flip_pieces), with the piece leaders' roots written when the
-// sweep is measured.
-template <int NT, bool kFew>
-__device__ __forceinline__ uint32_t resident_label(const Res &r, bool sweep, bool measure)
+// bond planes to final roots (every site's word at its root, the ROOT plane);
+// barriers between stages.  kSweep: the clusters are flipped, and in measured
+// sweeps the sites of the cluster most likely to be the largest are left in
+// the OH plane (free once the seams are done) and its root returned.
+template <int NT, bool kFew, bool kSweep>
+__device__ __forceinline__ uint32_t resident_label(const Res &r, bool measure)
 {
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     constexpr uint32_t nwarps = NT / 32;
+    // Words a warp takes at a time in the roots pass.  Measured on B200, cycles
+    // a site and SM with 1 / 2 / 4 / 8 words: L = 256 (1024 threads) 2.69 /
+    // 2.53 / 2.46 / 2.49, L = 64 (128) 3.18 / 3.04 / 2.98 / 3.11, L = 32 (one
+    // warp, many CTAs hide each other's latency) 5.70 / 5.92 / 6.12 / 6.26.
+    constexpr int kWords = NT <= 64 ? 1 : 4;
     unsigned short *list = r.LIST + warp * r.seg;
     phase_heads_open<kFew>(r.t, warp, nwarps);
     __syncthreads();
@@ -359,38 +362,28 @@ __device__ __forceinline__ uint32_t resident_label(const Res &r, bool sweep, boo
     __syncthreads();
     RBIM_PHASE_MARK(2);
     phase_seam(r, tid, NT);
-    for (uint32_t w = tid; w < r.t.g.NW; w += NT) r.t.ROOT[w] = 0u;
     __syncthreads();
     RBIM_PHASE_MARK(3);
     phase_seam_propagate(r, tid, NT);
     for (uint32_t i = tid; i < (r.t.g.L + 31u) / 32u; i += NT) r.t.SEAMV[i] = 0u;
     __syncthreads();
     RBIM_PHASE_MARK(4);
-    if (sweep && r.t.g.NW >= NT) {
-        // Every thread has a word: roots and flip in one pass over pieces.
-        const uint32_t nr = warp_sum(roots_flip_pieces(r.t, tid, NT));
-        __syncthreads();
-        RBIM_PHASE_MARK(11);
-        RBIM_PHASE_MARK(5);
-        return nr;
-    }
-    const uint32_t nr = warp_sum(phase_roots_flat(r.t, tid, NT));
-    __syncthreads();
-    RBIM_PHASE_MARK(11);
-    // Small lattices (fewer words than threads) flip site by site, which
-    // keeps every lane busy; this also leaves every site's word at its root.
-    phase_sites<Word16>(r.t, warp, nwarps, sweep, false);
+    const uint32_t likely = kSweep && measure ? likely_largest(r.t) : 0u;
+    roots_flip_sites<kSweep, kWords>(r.t, kSweep && measure ? r.t.OH : nullptr, likely, warp, nwarps);
     __syncthreads();
     RBIM_PHASE_MARK(5);
-    return nr;
+    return likely;
 }
 
 // Measurement of one sweep after resident_label: energy, magnetization,
 // n_clusters, S1, S2, |M_C1| and, with `second` (records requested), |M_C2|
-// (reference sw_sweep, src/rbim/swendsen_wang.py:146-172).  Ends with a
-// barrier.  Thread 0 returns the record in rec.
+// (reference sw_sweep, src/rbim/swendsen_wang.py:146-172).  The cluster rooted
+// at `likely`, whose sites are the set bits of OH, is counted and its
+// magnetization summed by popcounts; when it turns out to be the largest (as
+// it does whenever one cluster dominates) no pass for |M_C1| is needed.  Ends
+// with a barrier.  Thread 0 returns the record in rec.
 template <int NT>
-__device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, uint32_t nroots_warp,
+__device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, uint32_t likely,
                                                  long long rec[kRecLen], bool second)
 {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -399,36 +392,46 @@ __device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, u
     const Geom &g = t.g;
     unsigned short *u16 = t.uf.w;
 
-    // Energy and magnetization of the flipped spins.
-    uint32_t unsat = 0, downs = 0;
+    // Energy and magnetization of the flipped spins; clusters; size and down
+    // spins of the likely largest.
+    uint32_t unsat = 0, downs = 0, ncl = 0, in = 0, in_downs = 0;
     measure_energy(t, tid, NT, unsat, downs);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        unsat += __shfl_xor_sync(0xFFFFFFFFu, unsat, o);
-        downs += __shfl_xor_sync(0xFFFFFFFFu, downs, o);
+    for (uint32_t w = tid; w < g.NW; w += NT) {
+        const uint32_t c = t.OH[w];
+        ncl += __popc(t.ROOT[w]);
+        in += __popc(c);
+        in_downs += __popc(c & t.S[w]);
     }
+    unsat = __reduce_add_sync(0xFFFFFFFFu, unsat);
+    downs = __reduce_add_sync(0xFFFFFFFFu, downs);
+    ncl = __reduce_add_sync(0xFFFFFFFFu, ncl);
+    in = __reduce_add_sync(0xFFFFFFFFu, in);
+    in_downs = __reduce_add_sync(0xFFFFFFFFu, in_downs);
     if (lane == 0) {
         red.unsat[warp] = unsat;
         red.downs[warp] = downs;
-        red.roots[warp] = nroots_warp;
+        red.roots[warp] = ncl;
+        red.in[warp] = in;
+        red.in_downs[warp] = in_downs;
     }
     RBIM_PHASE_MARK(6);
     // Cluster sizes into the root words, on top of the index each root's word
     // holds (a root points at itself): afterwards a root's word is root + size
     // mod 2^16, which gives every size whenever there are two or more
     // clusters (each then below 65536); one cluster is the lattice.
-    count_pieces<false>(t, u16, warp, nwarps);
+    count_pieces<false>(t, u16, t.OH, warp, nwarps);
     __syncthreads();
     RBIM_PHASE_MARK(7);
     // Every warp sums the per-warp partials itself (no barrier needed after).
-    uint32_t unsat_t = lane < nwarps ? red.unsat[lane] : 0u, downs_t = lane < nwarps ? red.downs[lane] : 0u;
-    uint32_t ncl = lane < nwarps ? red.roots[lane] : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        unsat_t += __shfl_xor_sync(0xFFFFFFFFu, unsat_t, o);
-        downs_t += __shfl_xor_sync(0xFFFFFFFFu, downs_t, o);
-        ncl += __shfl_xor_sync(0xFFFFFFFFu, ncl, o);
-    }
+    const bool live = lane < nwarps;
+    const uint32_t unsat_t = __reduce_add_sync(0xFFFFFFFFu, live ? red.unsat[lane] : 0u);
+    const uint32_t downs_t = __reduce_add_sync(0xFFFFFFFFu, live ? red.downs[lane] : 0u);
+    ncl = __reduce_add_sync(0xFFFFFFFFu, live ? red.roots[lane] : 0u);
+    in = __reduce_add_sync(0xFFFFFFFFu, live ? red.in[lane] : 0u);
+    in_downs = __reduce_add_sync(0xFFFFFFFFu, live ? red.in_downs[lane] : 0u);
+    const long long M = (long long)g.N - 2ll * (long long)downs_t;
+    long long mc_total = M, mc2_total = 0;
+    uint32_t size1 = g.N, size2 = 0u;
     if (ncl > 1) {
         uint32_t k1 = 0, k2 = 0;
         for (uint32_t w = tid; w < g.NW; w += NT) {
@@ -437,7 +440,8 @@ __device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, u
                 const uint32_t b = __ffs(roots) - 1u;
                 roots &= roots - 1u;
                 const uint32_t r = (w << 5) + b;
-                top2_merge(k1, k2, ((((uint32_t)u16[r] - r) & 0xFFFFu) << 16) | (0xFFFFu - r), 0u);
+                const uint32_t size = r == likely ? in : ((uint32_t)u16[r] - r) & 0xFFFFu;
+                top2_merge(k1, k2, (size << 16) | (0xFFFFu - r), 0u);
             }
         }
         warp_top2(k1, k2);
@@ -446,24 +450,18 @@ __device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, u
             red.k2[warp] = k2;
         }
         __syncthreads();
-        if (warp == 0) {
-            uint32_t a1 = lane < nwarps ? red.k1[lane] : 0u, a2 = lane < nwarps ? red.k2[lane] : 0u;
-            warp_top2(a1, a2);
-            if (lane == 0) {
-                red.g1 = 0xFFFFu - (a1 & 0xFFFFu);
-                red.g2 = 0xFFFFu - (a2 & 0xFFFFu);
-                red.s1 = a1 >> 16;
-                red.s2 = a2 >> 16;
-            }
-        }
-        __syncthreads();
+        uint32_t a1 = live ? red.k1[lane] : 0u, a2 = live ? red.k2[lane] : 0u;
+        warp_top2(a1, a2);
         RBIM_PHASE_MARK(8);
-        const uint32_t g1 = red.g1, g2 = red.g2;
-        int mc = 0, mc2 = 0;
-        if (g.NW < NT) {
-            // Small lattices took the per-site path (every site's word holds
-            // its root): lanes are sites, which keeps all warps busy.  Two
-            // words per iteration keep two load chains in flight.
+        const uint32_t g1 = 0xFFFFu - (a1 & 0xFFFFu), g2 = 0xFFFFu - (a2 & 0xFFFFu);
+        size1 = a1 >> 16;
+        size2 = a2 >> 16;
+        mc_total = (long long)in - 2ll * (long long)in_downs;
+        if (g1 != likely || second) {
+            // Lanes are sites; every site's word holds its root (a root's own
+            // word its size, so roots are known by their ROOT bit).  Two words
+            // per iteration keep two load chains in flight.
+            int mc = 0, mc2 = 0;
             for (uint32_t w0 = warp; w0 < g.NW; w0 += 2u * nwarps) {
                 const uint32_t w1 = w0 + nwarps;
                 const uint32_t n0 = (w0 << 5) + lane, n1 = (w1 << 5) + lane;
@@ -482,63 +480,23 @@ __device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, u
                                           2 * (int)__popc(q1 & s1);
                 }
             }
-        } else {
-            // One lane per word, one test per run piece: the word of a piece's
-            // leader holds its root (its size counter when the leader is the
-            // root, recognised by its ROOT bit).  Measured faster on B200 than
-            // lanes-as-sites with the root read from each site's piece leader
-            // (15 k vs 24 k cycles per L = 256 sweep).
-            for (uint32_t w = tid; w < g.NW; w += NT) {
-                const uint32_t valid = g.valid(w);
-                uint32_t lead = piece_leaders(t, w, valid);
-                const uint32_t roots = t.ROOT[w], s = t.S[w];
-                const uint32_t nv = (uint32_t)__popc(valid);
-                while (lead) {
-                    const uint32_t b = __ffs(lead) - 1u;
-                    lead &= lead - 1u;
-                    const uint32_t end = lead ? (uint32_t)(__ffs(lead) - 1) : nv;
-                    const uint32_t n = (w << 5) + b;
-                    const uint32_t r = ((roots >> b) & 1u) ? n : (uint32_t)u16[n];
-                    const uint32_t pm = (end - b == 32u) ? 0xFFFFFFFFu : (((1u << (end - b)) - 1u) << b);
-                    const int m = (int)__popc(pm) - 2 * (int)__popc(pm & s);
-                    if (r == g1) mc += m;
-                    if (second && r == g2) mc2 += m;
-                }
+            if (lane == 0) {
+                red.mc[warp] = mc;
+                red.mc2[warp] = mc2;
             }
+            __syncthreads();
+            RBIM_PHASE_MARK(9);
+            mc_total = (int)__reduce_add_sync(0xFFFFFFFFu, (uint32_t)(live ? red.mc[lane] : 0));
+            mc2_total = (int)__reduce_add_sync(0xFFFFFFFFu, (uint32_t)(live ? red.mc2[lane] : 0));
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mc += __shfl_xor_sync(0xFFFFFFFFu, mc, o);
-            mc2 += __shfl_xor_sync(0xFFFFFFFFu, mc2, o);
-        }
-        if (lane == 0) {
-            red.mc[warp] = mc;
-            red.mc2[warp] = mc2;
-        }
-        __syncthreads();
-        RBIM_PHASE_MARK(9);
-    } else if (tid == 0) {
-        // One cluster covers the lattice.
-        red.g1 = 0;
-        red.s1 = g.N;
-        red.s2 = 0;
     }
-    const long long M = (long long)g.N - 2ll * (long long)downs_t;
     if (tid == 0) {
-        long long mc_total = M, mc2_total = 0;
-        if (ncl > 1) {
-            mc_total = 0;
-            for (uint32_t i = 0; i < nwarps; ++i) {
-                mc_total += red.mc[i];
-                mc2_total += red.mc2[i];
-            }
-        }
         rec[0] = 2ll * (long long)unsat_t - 2ll * (long long)g.N;
         rec[1] = M;
         rec[2] = ncl;
-        rec[3] = red.s1;
+        rec[3] = size1;
         rec[4] = mc_total < 0 ? -mc_total : mc_total;
-        rec[5] = red.s2;
+        rec[5] = size2;
         rec[6] = mc2_total < 0 ? -mc2_total : mc2_total;
         rec[7] = red.wrap & 1;
         rec[8] = (red.wrap >> 1) & 1;
@@ -611,11 +569,11 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
             phase_activate<Word16>(t, make_rng(ch.key, sweep, ch.thr), warp, nwarps, tid, NT);
             __syncthreads();
             RBIM_PHASE_MARK(0);
-            const uint32_t nr = resident_label<NT, NT >= 512 && LC == 0>(res, true, measure);
+            const uint32_t likely = resident_label<NT, NT >= 512 && LC == 0, true>(res, measure);
             if (measure) {
                 long long rec[kRecLen];
                 const bool want_rec = records && ch.rec_off >= 0;
-                resident_measure<NT>(res, red, nr, rec, want_rec);
+                resident_measure<NT>(res, red, likely, rec, want_rec);
                 if (tid == 0) {
                     const long long idx = (long long)(sweep - (uint64_t)ch.n_therm);
                     const long long bin = idx / ch.sweeps_per_bin;
@@ -696,7 +654,7 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
         }
     }
     __syncthreads();
-    resident_label<NT, false>(res, false, false);
+    (void)resident_label<NT, false, false>(res, false);
     // Exclusive prefix of root counts over words -> FLIP plane (rank base).
     const uint32_t per = (g.NW + NT - 1u) / NT;
     const uint32_t w0 = tid * per, w1 = min(g.NW, w0 + per);

@@ -104,14 +104,8 @@ __device__ __forceinline__ void tile_activate(const Lat<Word16> &t, uint32_t *YS
     }
 }
 
-// Root of tile site x after the open labelling's roots pass: every parent is
-// a run head and every head points at its root.
-__device__ __forceinline__ uint32_t tile_root(const unsigned short *uf, uint32_t x)
-{
-    const uint32_t p = uf[x];
-    const uint32_t q = uf[p];
-    return q == p ? p : q;
-}
+// Root of tile site x after the roots pass: every site's word holds it.
+__device__ __forceinline__ uint32_t tile_root(const unsigned short *uf, uint32_t x) { return uf[x]; }
 
 template <int NT>
 __device__ __forceinline__ void tile_energy(const Lat<Word16> &t, const Tile &tl, const uint32_t *gJH,
