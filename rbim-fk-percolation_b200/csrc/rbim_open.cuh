@@ -86,6 +86,7 @@ struct UpBonds {
     uint32_t heads;   // run heads of the word
     uint32_t above;   // run heads of the sites n - L
     uint32_t link;    // bonds that link their run's head to the run above
+    uint32_t linked;  // those heads
     uint32_t need;    // bonds left to the unions
 };
 
@@ -97,6 +98,7 @@ __device__ __forceinline__ UpBonds up_bonds(const Lat<Word16> &t, uint32_t w)
     r.heads = head_mask(t.OV, w, valid);
     r.above = 0u;
     r.link = 0u;
+    r.linked = 0u;
     r.need = 0u;
     if ((w << 5) + 31u < g.L) return r;  // the first row has no up-bonds
     // Bits u - 1 .. u + 31 of OH and u - 1 .. u + 30 of OV (words before the
@@ -119,6 +121,9 @@ __device__ __forceinline__ UpBonds up_bonds(const Lat<Word16> &t, uint32_t w)
     const uint32_t in_run = ~r.heads;
     r.link = k & ~fill_up((k << 1) & in_run, in_run);
     r.need = c & ~r.link;
+    // From each link down its run to the head, with the bits reversed.
+    const uint32_t back = __brev(r.link), run = __brev(in_run);
+    r.linked = r.heads & __brev(back | (fill_up(back & run, run) << 1));
     return r;
 }
 
@@ -135,38 +140,25 @@ __device__ __forceinline__ Band warp_band(uint32_t NW, uint32_t warp, uint32_t n
     return {first, min(NW, first + per)};
 }
 
-// Parent of one site of a word: the last run head up to it (`le`: the bits up
-// to the site's), or for a head whose run has a link the head above the link,
-// or that head's own parent when it was written before (`done` sites from
-// band0 on).  h, link, above: the word's UpBonds; before: 1 + the last head
-// before the word; n0: the word's first site.
-__device__ __forceinline__ uint32_t open_parent(const UF<Word16> &uf, uint32_t h, uint32_t before, uint32_t link,
-                                                uint32_t above, uint32_t n0, uint32_t le, uint32_t L, uint32_t band0,
-                                                uint32_t done)
+// Parent of one site of a word (`le`: the bits up to the site's): the last run
+// head of the word up to it, or for a head with a link the head above the
+// link, or that head's own parent when it was written before (`done` sites
+// from band0 on).  A site whose run began in an earlier word points at the
+// word's predecessor n0 - 1, which is in its run.  n0: the word's first site.
+__device__ __forceinline__ uint32_t open_parent(const UF<Word16> &uf, const UpBonds &ub, uint32_t n0, uint32_t le,
+                                                uint32_t L, uint32_t band0, uint32_t done)
 {
-    const uint32_t f = link & ~(le >> 1);  // the lowest of f is the link of a run headed here ...
-    const uint32_t upto = f ^ (f - 1u);
-    const bool linked = f && (h & (le ^ (le >> 1))) && !(h & upto & ~le);  // ... if no other head comes before
-    const uint32_t m = linked ? above & upto : h & le;
+    const uint32_t f = ub.link & ~(le >> 1);  // a linked head's link is the lowest of f
+    const bool linked = ub.linked & (le ^ (le >> 1));
+    const uint32_t m = linked ? ub.above & (f ^ (f - 1u)) : ub.heads & le;
     uint32_t p = (linked ? n0 - L : n0) + 31u - __clz(m);
-    if (!m) p = before - 1u;
     if (linked && p - band0 < done) p = uf.ld(p);
     return p;
 }
 
-// 1 + the last run head before word w (0: there is none).
-__device__ __forceinline__ uint32_t last_head_before(const Lat<Word16> &t, uint32_t w)
-{
-    // Site 0 always heads a run, so this walk back ends.
-    while (w-- > 0) {
-        const uint32_t h = head_mask(t.OV, w, 0xFFFFFFFFu);
-        if (h) return (w << 5) + 32u - __clz(h);
-    }
-    return 0u;
-}
-
 // (b) Union-find initialisation: every site points at the head of its run of
-// occupied y-bonds, and a run head with an occupied x-bond to the row above at
+// occupied y-bonds (through the last site of the word before, when the run
+// began there), and a run head with an occupied x-bond to the row above at
 // the run above, with plain stores (a head takes one such link, to a smaller
 // site, so nothing can race).  A warp writes its band of consecutive words two
 // by two (lanes 0-15 one word, 16-31 the next, two sites a lane, one 32-bit
@@ -176,9 +168,10 @@ __device__ __forceinline__ uint32_t last_head_before(const Lat<Word16> &t, uint3
 // another warp meanwhile) takes the upper head itself.  The bonds that are
 // left go to NEED for the unions: at L = 256 about 9 k of 28 k bonds.
 //
-// Per group of 32 words, lane j finds the heads and up-bonds of word j, and a
-// max-scan over the lanes gives every word the last head before it.  kFew: for
-// launches whose warps may have a single word, which all lanes then look at.
+// Per group of 32 words, lane j finds the heads and up-bonds of word j.  Bound
+// by the integer pipe, so what can be done on whole words is done there.  kFew:
+// for launches whose warps may have a single word, which all lanes then look
+// at.
 template <bool kFew>
 __device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t warp, uint32_t nwarps)
 {
@@ -189,12 +182,11 @@ __device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t 
         const uint32_t w = band.first, n0 = w << 5;
         const UpBonds ub = up_bonds(t, w);
         if (lane == 0) t.NEED[w] = ub.need;
-        const uint32_t before = (ub.heads & 1u) ? 0u : last_head_before(t, w);
-        const uint32_t p = open_parent(t.uf, ub.heads, before, ub.link, ub.above, n0, mask_le(lane), g.L, 0u, 0u);
+        const uint32_t p = open_parent(t.uf, ub, n0, mask_le(lane), g.L, 0u, 0u);
         if (n0 + lane < g.N) t.uf.st(n0 + lane, (unsigned short)p);
         return;
     }
-    const uint32_t band0 = band.first << 5, b0 = 2u * (lane & 15u), le0 = mask_le(b0);
+    const uint32_t band0 = band.first << 5, b0 = 2u * (lane & 15u), le0 = mask_le(b0), le1 = 2u * le0 + 1u;
     for (uint32_t base = band.first; base < band.end; base += 32u) {
         const uint32_t wj = base + lane;
         UpBonds ub{};
@@ -202,27 +194,18 @@ __device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t 
             ub = up_bonds(t, wj);
             t.NEED[wj] = ub.need;
         }
-        const uint32_t h = ub.heads;
-        const uint32_t pre = lane == 0 && !(h & 1u) ? last_head_before(t, base) : 0u;
         const uint32_t count = min(32u, band.end - base);
-        uint32_t incl = max(h ? (wj << 5) + 32u - __clz(h) : 0u, pre);
-        for (uint32_t o = 1; o < count; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl = max(incl, v);
-        }
-        // Last head before word j: the scan of lanes < j, or pre for j = 0.
-        uint32_t before = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
-        if (lane == 0) before = pre;
         for (uint32_t j = 0; j < count; j += 2u) {
             const uint32_t jj = j + (lane >> 4);
-            const uint32_t hj = __shfl_sync(0xFFFFFFFFu, h, jj);
-            const uint32_t cj = __shfl_sync(0xFFFFFFFFu, before, jj);
-            const uint32_t lj = __shfl_sync(0xFFFFFFFFu, ub.link, jj);
-            const uint32_t aj = __shfl_sync(0xFFFFFFFFu, ub.above, jj);
+            UpBonds w;
+            w.heads = __shfl_sync(0xFFFFFFFFu, ub.heads, jj);
+            w.above = __shfl_sync(0xFFFFFFFFu, ub.above, jj);
+            w.link = __shfl_sync(0xFFFFFFFFu, ub.link, jj);
+            w.linked = __shfl_sync(0xFFFFFFFFu, ub.linked, jj);
             const uint32_t n0 = (base + jj) << 5, n = n0 + b0;
             const uint32_t done = ((base + j) << 5) - band0;  // sites of the band written in earlier steps
-            const uint32_t p0 = open_parent(t.uf, hj, cj, lj, aj, n0, le0, g.L, band0, done);
-            const uint32_t p1 = open_parent(t.uf, hj, cj, lj, aj, n0, 2u * le0 + 1u, g.L, band0, done);
+            const uint32_t p0 = open_parent(t.uf, w, n0, le0, g.L, band0, done);
+            const uint32_t p1 = open_parent(t.uf, w, n0, le1, g.L, band0, done);
             if (jj < count) {
                 if (n + 1u < g.N)
                     t.uf.st2(n, p0 | (p1 << 16));
