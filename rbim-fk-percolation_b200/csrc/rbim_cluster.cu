@@ -193,6 +193,7 @@ __device__ __forceinline__ Ctx make_ctx(unsigned char *smem, const ClusterLayout
     t.ROOT = (uint32_t *)(smem + ly.off_ROOT);
     t.NEED = t.ROOT;  // read by the unions, before the roots are recorded
     t.RE = nullptr;
+    t.inv = 0u;
     t.SEAMV = nullptr;
     t.wrap = &red.wrap;
     t.err = &red.err;

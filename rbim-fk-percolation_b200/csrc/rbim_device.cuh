@@ -117,10 +117,11 @@ struct Geom {
         return (n0 + 32u <= N) ? 0xFFFFFFFFu : ((1u << (N - n0)) - 1u);
     }
     // Bits whose site has y == L-1 (row ends) among sites 32w .. 32w+31.
-    __device__ __forceinline__ uint32_t row_end(uint32_t w) const
+    __device__ __forceinline__ uint32_t row_end(uint32_t w) const { return row_end(w, (w << 5) % L); }
+    // The same with the y of site 32w known.
+    __device__ __forceinline__ uint32_t row_end(uint32_t w, uint32_t y) const
     {
-        const uint32_t n0 = w << 5;
-        uint32_t p = (L - 1u) - (n0 % L);
+        uint32_t p = (L - 1u) - y;
         uint32_t m = 0;
         for (; p < 32u; p += L) m |= 1u << p;
         return m & valid(w);

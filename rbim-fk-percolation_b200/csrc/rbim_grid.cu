@@ -393,6 +393,7 @@ __device__ __forceinline__ GTile make_gtile(unsigned char *smem, const GridLayou
     t.FLIP = (uint32_t *)(smem + ly.off_FLIP);
     t.ROOT = (uint32_t *)(smem + ly.off_ROOT);
     t.RE = nullptr;
+    t.inv = 0u;
     t.SEAMV = nullptr;
     t.wrap = &red.wrap;
     t.err = &red.err;

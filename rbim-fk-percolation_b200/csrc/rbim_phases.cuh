@@ -31,10 +31,19 @@ struct Lat {
     uint32_t *FLIP, *ROOT;
     uint32_t *NEED;        // open labelling: up-bonds left to the unions (may share ROOT's words)
     const uint32_t *RE;    // row-end masks per word (Geom::row_end), or null to compute them
+    uint32_t inv;          // ceil(2^32 / L) for N <= 65536, or 0 to divide
     int *wrap;             // bit 0 wrap_x, bit 1 wrap_y
     int *err;
     uint32_t cap;          // bound on the steps of one walk (N + 64 unless a chain's walk_cap lowers it)
-    __device__ __forceinline__ uint32_t row_end(uint32_t w) const { return RE ? RE[w] : g.row_end(w); }
+    // Row of site n.  With n < 2^16 and L <= 2^8 the error of the reciprocal,
+    // below L / 2^32 a site, is too small to reach the next row.
+    __device__ __forceinline__ uint32_t row(uint32_t n) const { return inv ? __umulhi(n, inv) : n / g.L; }
+    __device__ __forceinline__ uint32_t row_end(uint32_t w) const
+    {
+        if (RE) return RE[w];
+        const uint32_t n0 = w << 5;
+        return g.row_end(w, n0 - row(n0) * g.L);
+    }
 };
 
 struct SweepRng {
@@ -196,11 +205,10 @@ __device__ __forceinline__ void draw_group(const SweepRng &rng, const BondDraw &
 // warp handling chunk c draws Philox block 32c + i, whose word s holds the
 // 16-bit draws of the horizontal (low half) and vertical (high half) bond of
 // site 128c + 32s + i, i.e. bit i of the chunk's word s, so that each ballot
-// is one word of the occupied-bond planes.  A warp takes a group of G
-// consecutive words (G = 32, eight chunks, while every warp still gets a
-// group): lane j forms the satisfied masks of word j of the group -- every
-// lane busy, coalesced loads -- and keeps the ballots of its own word.  SEAMV
-// must be zero on entry.
+// is one word of the occupied-bond planes.  The chunks are split evenly in
+// consecutive ones per warp, which takes them in groups of eight: lane j
+// keeps the ballots of word j of the group and forms its satisfied masks
+// (coalesced loads).  SEAMV must be zero on entry.
 template <class WT>
 __device__ __forceinline__ void phase_activate_bonds(const Lat<WT> &t, const SweepRng &rng, uint32_t warp,
                                                      uint32_t nwarps)
@@ -208,17 +216,15 @@ __device__ __forceinline__ void phase_activate_bonds(const Lat<WT> &t, const Swe
     const uint32_t lane = threadIdx.x & 31u;
     const Geom &g = t.g;
     Plane S{t.S};
-    uint32_t G = 32u;
-    while (G > 4u && G * nwarps > g.NW) G >>= 1;
-    const uint32_t ngroups = (g.NW + G - 1u) / G;
-    const uint32_t nchunks = (g.NW + 3u) >> 2;
+    const uint32_t nchunks = (g.NW + 3u) >> 2, per = (nchunks + nwarps - 1u) / nwarps;
+    const uint32_t end = min(nchunks, (warp + 1u) * per);
     const BondDraw draw = make_bond_draw(rng);
-    for (uint32_t grp = warp; grp < ngroups; grp += nwarps) {
-        const uint32_t c0 = grp * (G >> 2);
+    for (uint32_t c0 = warp * per; c0 < end; c0 += 8u) {
+        const uint32_t nch = min(8u, end - c0);
         uint32_t oh, ov;
-        draw_group(rng, draw, 32u * c0 + lane, min(G >> 2, nchunks - c0), lane, oh, ov);
-        const uint32_t w = grp * G + lane;
-        if (lane < G && w < g.NW) {
+        draw_group(rng, draw, 32u * c0 + lane, nch, lane, oh, ov);
+        const uint32_t w = 4u * c0 + lane;
+        if (lane < 4u * nch && w < g.NW) {
             const uint32_t re = t.row_end(w), v = g.valid(w), s = S(w);
             oh &= ~(s ^ xnext_word(S, w, g) ^ t.JH[w]) & v;
             ov &= ~(s ^ ynext_word(S, w, g, re) ^ t.JV[w]) & v;
@@ -228,7 +234,7 @@ __device__ __forceinline__ void phase_activate_bonds(const Lat<WT> &t, const Swe
             while (seam) {
                 const uint32_t b = __ffs(seam) - 1u;
                 seam &= seam - 1u;
-                const uint32_t x = ((w << 5) + b) / g.L;
+                const uint32_t x = t.row((w << 5) + b);
                 atomicOr(t.SEAMV + (x >> 5), 1u << (x & 31u));
             }
         }

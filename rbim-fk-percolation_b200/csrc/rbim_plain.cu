@@ -169,6 +169,7 @@ __device__ __forceinline__ Lat<Word64> plain_lat(const PlainArgs &a)
     t.ROOT = a.ws.ROOT;
     t.SEAMV = a.ws.SEAMV;
     t.RE = nullptr;
+    t.inv = 0u;
     t.wrap = &a.ws.sc->wrap;
     t.err = &a.ws.sc->err;
     // A descriptor's walk_cap > 0 lowers the walk bound (a test hook).
@@ -446,6 +447,7 @@ __device__ __forceinline__ Lat<Word64> label_lat(const PlainWs &ws, uint32_t L)
     t.ROOT = ws.ROOT;
     t.SEAMV = ws.SEAMV;
     t.RE = nullptr;
+    t.inv = 0u;
     t.wrap = &ws.sc->wrap;
     t.err = &ws.sc->err;
     t.cap = t.g.N + 64u;

@@ -33,10 +33,11 @@ constexpr uint32_t kMaxResidentSites = 65536;  // 16-bit parents
 // kernels' static shared scratch.
 constexpr size_t kMaxSmem = 227 * 1024 - 8 * 1024;
 constexpr uint32_t kHashEmpty = 0xFFFFFFFFu;
-// Shared memory of one SM, and an allowance for a CTA's static shared scratch
-// and the per-CTA reservation, when deciding how many CTAs fit an SM.
+// Shared memory of one SM, and what a CTA takes beside its dynamic part: the
+// per-CTA reservation of 1 KB and the static scratch (Red<512>, 0.8 KB), when
+// deciding how many CTAs fit an SM.
 constexpr size_t kSmemPerSm = 228 * 1024;
-constexpr size_t kStaticSmem = 2 * 1024;
+constexpr size_t kStaticSmem = 1024 + 832;
 
 __host__ __device__ constexpr size_t align16(size_t v) { return (v + 15) & ~size_t(15); }
 
@@ -123,8 +124,12 @@ __host__ __device__ constexpr ResidentLayout resident_layout_c(uint32_t l_max, i
     off += plane;
     ly.off_ROOT = off;
     off += plane;
+    // Row-end masks, for the CTA sizes of the small lattices: several rows end
+    // in a word there (masks computed each sweep cost 3 % at L = 64, 10 % at
+    // L = 40). Larger CTAs compute them: without the plane a fourth CTA of 256
+    // threads fits an SM at L = 127 and 128 (-8 %).
     ly.off_RE = off;
-    off += plane;
+    if (threads <= 128) off += plane;
     ly.off_SEAMV = off;
     off = align16(off + 4ull * (((l_max + 31u) / 32u) + 4u));
     ly.off_HK = off;
@@ -162,13 +167,17 @@ int resident_default_threads(int l_max)
     // At 64 registers a thread an SM holds 1024 of this kernel's threads
     // whatever the CTA size, and several small CTAs per SM hide each other's
     // barrier waits better than one large one; so the CTA is as small as the
-    // lattice allows before its per-thread work grows long.  Measured on
-    // B200: 32 threads (one warp) up to L = 32 (against 64: +36 % at L = 16,
-    // +7 % at 24, +17 % at 32), 128 up to 64, 256 up to 96, then 512 while
-    // two CTAs' shared memory fits an SM (up to L = 180), then 1024.
+    // lattice allows before its per-thread work grows long and its shared
+    // memory keeps threads off the SM.  Measured on B200, cycles a site and SM
+    // with half / this / twice the threads: L = 32: - / 4.4 / 4.7; L = 40: 5.0
+    // / 4.5 / 5.0; L = 48: 4.4 / 4.2 / 5.0; L = 64: 3.3 / 2.7 / 3.4; L = 72: 3.4
+    // / 3.1 / 4.7; L = 124: 3.2 / 2.3 / 2.8; L = 144: 3.4 / 2.7 / 3.4; L = 181:
+    // 3.2 / 2.4 / 2.7, and above, where one CTA of 512 threads would have the
+    // SM to itself, L = 192: 5.3 / 3.6 / 2.9.
     if (l_max <= 32) return 32;
+    if (l_max <= 44) return 64;
     if (l_max <= 64) return 128;
-    if (l_max <= 96) return 256;
+    if (l_max <= 128) return 256;
     if (2 * (resident_layout_c((uint32_t)l_max, 512).bytes + kStaticSmem) <= kSmemPerSm) return 512;
     return 1024;
 }
@@ -222,7 +231,8 @@ __device__ __forceinline__ Res make_res(unsigned char *smem, const ResidentLayou
     t.FLIP = (uint32_t *)(smem + ly.off_FLIP);
     t.ROOT = (uint32_t *)(smem + ly.off_ROOT);
     t.NEED = t.ROOT;  // read by the unions, before the roots are recorded
-    t.RE = (const uint32_t *)(smem + ly.off_RE);
+    t.RE = NT <= 128 ? (const uint32_t *)(smem + ly.off_RE) : nullptr;
+    t.inv = NT <= 128 ? 0u : 0xFFFFFFFFu / L + 1u;
     t.SEAMV = (uint32_t *)(smem + ly.off_SEAMV);
     t.wrap = &red.wrap;
     t.err = &red.err;
@@ -236,12 +246,13 @@ __device__ __forceinline__ Res make_res(unsigned char *smem, const ResidentLayou
     return r;
 }
 
-// Row-end masks of the lattice (computed once per chain, so that the sweep
-// needs no integer division).
-__device__ __forceinline__ void init_row_ends(const Lat<Word16> &t, uint32_t tid, uint32_t nthreads)
+// The row-end masks (once per chain).
+template <int NT>
+__device__ __forceinline__ void init_row_ends(const Lat<Word16> &t, uint32_t tid)
 {
+    if (NT > 128) return;
     uint32_t *re = const_cast<uint32_t *>(t.RE);
-    for (uint32_t w = tid; w < t.g.NW; w += nthreads) re[w] = t.g.row_end(w);
+    for (uint32_t w = tid; w < t.g.NW; w += NT) re[w] = t.g.row_end(w);
 }
 
 __device__ __forceinline__ uint32_t hash_insert(const Res &r, uint32_t key, int *err)
@@ -555,7 +566,7 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
                 ((uint4 *)t.JV)[i] = gv[i];
             }
             for (uint32_t i = tid; i < (L + 31u) / 32u; i += NT) t.SEAMV[i] = 0u;
-            init_row_ends(t, tid, NT);
+            init_row_ends<NT>(t, tid);
         }
         const uint64_t t_end = (uint64_t)ch.n_therm + (uint64_t)ch.n_bins * (uint64_t)ch.sweeps_per_bin;
         uint64_t sweep = ch.sweep;
@@ -632,7 +643,7 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
     const Geom g = t.g;
     const uint8_t *o = occ + lat * 2ull * g.N;
     for (uint32_t i = tid; i < (L + 31u) / 32u; i += NT) t.SEAMV[i] = 0u;
-    init_row_ends(t, tid, NT);
+    init_row_ends<NT>(t, tid);
     __syncthreads();
     for (uint32_t w = tid; w < g.NW; w += NT) {
         uint32_t h = 0, v = 0;
@@ -642,14 +653,14 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
             h |= (o[2ull * n] ? 1u : 0u) << b;
             v |= (o[2ull * n + 1] ? 1u : 0u) << b;
         }
-        const uint32_t re = g.row_end(w);
+        const uint32_t re = t.row_end(w);
         t.OH[w] = h;
         t.OV[w] = v & ~re;
         uint32_t seam = v & re;
         while (seam) {
             const uint32_t b = __ffs(seam) - 1u;
             seam &= seam - 1u;
-            const uint32_t x = ((w << 5) + b) / L;
+            const uint32_t x = t.row((w << 5) + b);
             atomicOr(t.SEAMV + (x >> 5), 1u << (x & 31u));
         }
     }
@@ -715,9 +726,9 @@ cudaError_t launch_sweeps_lc(const rbim_chain_t *chains, int n_chains, int l_max
     return cudaGetLastError();
 }
 
-// Size classes with a compile-time layout, at their default thread counts:
-// 128 < L <= 256 (1024 threads), 96 < L <= 128 and 128 < L <= 176 (512),
-// 64 < L <= 96 (256).  Below L = 64 (CTAs of 64 and 128 threads) the
+// Size classes with a compile-time layout:
+// 128 < L <= 256 (1024 threads), 96 < L <= 128 and 128 < L <= 176 (512), 64 <
+// L <= 96 and 96 < L <= 128 (256).  Below L = 64 (CTAs of 64 and 128 threads) the
 // run-time layout measured 5-7% faster than a compile-time one on B200.
 template <int NT>
 cudaError_t launch_sweeps_nt(const rbim_chain_t *chains, int n_chains, int l_max, uint32_t *spin_pool,
@@ -741,6 +752,9 @@ cudaError_t launch_sweeps_nt(const rbim_chain_t *chains, int n_chains, int l_max
         if (l_max > 64 && l_max <= 96)
             return launch_sweeps_lc<NT, 96>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
                                             n_sweeps, grid, queue, status, stream);
+        if (l_max > 96 && l_max <= 128)
+            return launch_sweeps_lc<NT, 128>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec,
+                                             n_sweeps, grid, queue, status, stream);
     }
     return launch_sweeps_lc<NT, 0>(chains, n_chains, l_max, spin_pool, coupling_pool, acc_i, acc_f, rec, n_sweeps,
                                    grid, queue, status, stream);

@@ -63,17 +63,15 @@ __device__ __forceinline__ void tile_activate(const Lat<Word16> &t, uint32_t *YS
     const uint32_t chunk0 = tl.b >> 7;
     const uint32_t last = tl.Tc - 1u;
     const bool end_is_row_end = ((tl.b + tl.Tc) % tl.L) == 0u;
-    // Groups of G consecutive words, as in phase_activate_bonds.
-    uint32_t G = 32u;
-    while (G > 4u && G * nwarps > g.NW) G >>= 1;
-    const uint32_t ngroups = (g.NW + G - 1u) / G;
+    // Chunks per warp and groups of eight, as in phase_activate_bonds.
+    const uint32_t per = (nchunks + nwarps - 1u) / nwarps, end = min(nchunks, (warp + 1u) * per);
     const BondDraw draw = make_bond_draw(rng);
-    for (uint32_t grp = warp; grp < ngroups; grp += nwarps) {
-        const uint32_t c0 = grp * (G >> 2);
+    for (uint32_t c0 = warp * per; c0 < end; c0 += 8u) {
+        const uint32_t nch = min(8u, end - c0);
         uint32_t oh, ov;
-        draw_group(rng, draw, 32u * (chunk0 + c0) + lane, min(G >> 2, nchunks - c0), lane, oh, ov);
-        const uint32_t w = grp * G + lane;
-        if (lane < G && w < g.NW) {
+        draw_group(rng, draw, 32u * (chunk0 + c0) + lane, nch, lane, oh, ov);
+        const uint32_t w = 4u * c0 + lane;
+        if (lane < 4u * nch && w < g.NW) {
             const uint32_t v = g.valid(w), re = tile_row_end(tl, w, v), s = t.S[w];
             oh &= ~(s ^ extract_nowrap(t.S, (w << 5) + tl.L) ^ gJH[w]) & v;
             ov &= ~(s ^ tile_ynext(t.S, w, re, tl.L, front) ^ gJV[w]) & v;

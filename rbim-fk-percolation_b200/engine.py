@@ -290,12 +290,13 @@ class ChainSet:
 
         # Descriptor slots grouped by launch bucket: resident lattices by size
         # class, cluster lattices by CTAs per cluster, then those only the plain
-        # engine takes (engine_buckets).
+        # engine takes (engine_buckets); within a bucket the largest lattices
+        # first, so that no long run starts at the end of the work queue.
         with torch.cuda.device(self.device):
             r_max = _native.resident_max_l()
             c_max = _native.cluster_max_l()
             keys = _native.engine_buckets(Ls, r_max, c_max)
-        order = np.array(sorted(range(self.n), key=lambda i: keys[i]), dtype=np.int64)
+        order = np.array(sorted(range(self.n), key=lambda i: (keys[i], -self.specs[i].L)), dtype=np.int64)
         self.slot = np.empty(self.n, dtype=np.int64)
         self.slot[order] = np.arange(self.n)
         self.buckets = []  # (kind, first slot, count, l_max)

@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("L,threads", [(3, 32), (3, 1024), (6, 256), (11, 64), (16, 32), (16, 1024), (31, 64), (32, 512),
                                        (33, 32), (33, 1024), (47, 128), (63, 1024), (65, 256), (96, 256), (97, 512),
-                                       (128, 512), (129, 1024), (181, 1024), (255, 1024), (256, 1024)])
+                                       (120, 256), (127, 256), (128, 256), (128, 512), (129, 1024), (181, 512),
+                                       (184, 512), (185, 1024), (255, 1024), (256, 1024)])
 def test_resident_bands_match_oracle(rb, orc, L, threads):
     rng = np.random.default_rng(100 * L + threads)
     # Hot and critical, nearly full (long runs, one cluster), nearly empty, and frustrated.
