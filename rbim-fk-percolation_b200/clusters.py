@@ -83,25 +83,64 @@ def label_and_wrap_many(active: np.ndarray, L: int, device=None):
     """
     torch = _torch()
     dev = require_cuda(device)
-    a = np.ascontiguousarray(np.asarray(active).reshape(-1, 2 * L * L), dtype=np.uint8)
+    a = np.asarray(active)
+    if a.dtype == np.bool_:
+        a = np.ascontiguousarray(a).view(np.uint8)  # a boolean is a byte of 0 or 1
+    a = np.ascontiguousarray(a.reshape(-1, 2 * L * L), dtype=np.uint8)
     n = a.shape[0]
     lib = _native.lib()
     occ = torch.from_numpy(a).to(dev)
     labels = torch.empty((n, L * L), dtype=torch.int32, device=dev)
-    ncl = torch.empty(n, dtype=torch.int32, device=dev)
-    wraps = torch.empty((n, 2), dtype=torch.uint8, device=dev)
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    # Status word, cluster counts and wrap flags, back in one copy.
+    meta = torch.zeros(4 + 4 * n + 2 * n, dtype=torch.uint8, device=dev)
     nbytes = int(lib.rbim_label_wrap_workspace_bytes(L))
     ws = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=dev)
-    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    p = ctypes.c_void_p
     with torch.cuda.device(dev):
-        rc = lib.rbim_label_wrap(L, n, p(occ), p(labels), p(ncl), p(wraps), p(status), p(ws), ws.numel(), _stream(dev))
-    _native.check(rc, "rbim_label_wrap")
-    st = int(status.item())
-    if st:
-        raise _native.RbimError(f"rbim_label_wrap device status {st:#x}")
-    return (ncl.cpu().numpy().astype(np.int64), labels.cpu().numpy().astype(np.int64),
-            wraps.cpu().numpy().astype(bool))
+        rc = lib.rbim_label_wrap(L, n, p(occ.data_ptr()), p(labels.data_ptr()), p(meta.data_ptr() + 4),
+                                 p(meta.data_ptr() + 4 + 4 * n), p(meta.data_ptr()), p(ws.data_ptr()), ws.numel(),
+                                 _stream(dev))
+        _native.check(rc, "rbim_label_wrap")
+        m = meta.cpu().numpy()
+        st = int(m[:4].view(np.int32)[0])
+        if st:
+            raise _native.RbimError(f"rbim_label_wrap device status {st:#x}")
+        wide = _to_host_int64(labels)
+    return m[4: 4 + 4 * n].view(np.int32).astype(np.int64), wide, m[4 + 4 * n:].reshape(n, 2).astype(bool)
+
+
+#: Elements of one pinned staging buffer of :func:`_to_host_int64` (4 MB).
+_STAGE = 1 << 20
+
+
+def _to_host_int64(t) -> np.ndarray:
+    """A device int32 tensor as a host int64 array.
+
+    Chunks go through two pinned buffers (at most 8 MB a call, from torch's
+    caching host allocator), and torch widens one on the host's threads while
+    the next is copied.  Against a pageable copy of the whole tensor and
+    numpy's widening, 16.8 MB of labels take 2.2 ms instead of 9.4 ms: both of
+    those touch their fresh pages from one thread.
+    """
+    torch = _torch()
+    flat = t.view(-1)
+    total = flat.numel()
+    out = torch.empty(total, dtype=torch.int64)
+    size = min(_STAGE, max(total, 1))
+    stage = [torch.empty(size, dtype=torch.int32, pin_memory=True) for _ in range(2 if total > size else 1)]
+    ready = [torch.cuda.Event() for _ in stage]
+    stream = torch.cuda.current_stream(t.device)
+    chunks = [(k, min(k + size, total)) for k in range(0, total, size)]
+    for i in range(len(chunks) + 1):
+        if i < len(chunks):
+            lo, hi = chunks[i]
+            stage[i % 2][: hi - lo].copy_(flat[lo:hi], non_blocking=True)
+            ready[i % 2].record(stream)
+        if i > 0:
+            lo, hi = chunks[i - 1]
+            ready[(i - 1) % 2].synchronize()
+            out[lo:hi].copy_(stage[(i - 1) % 2][: hi - lo])
+    return out.numpy().reshape(t.shape)
 
 
 def label_and_wrap(active: np.ndarray, lattice: Lattice) -> Tuple[int, np.ndarray, bool, bool]:

@@ -713,9 +713,11 @@ cudaError_t launch_sweeps_lc(const rbim_chain_t *chains, int n_chains, int l_max
         int per_sm = 0, sms = 0, dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident_sweeps<NT, LC>, NT, ly.bytes);
-        if (e != cudaSuccess) return e;
-        grid = std::max(1, per_sm) * sms;
+        if (n_chains > sms) {
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident_sweeps<NT, LC>, NT, ly.bytes);
+            if (e != cudaSuccess) return e;
+        }
+        grid = std::max(1, per_sm) * std::max(1, sms);
     }
     grid = std::min(grid, n_chains);
     e = cudaMemsetAsync(queue, 0, sizeof(int), stream);

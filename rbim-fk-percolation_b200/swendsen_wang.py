@@ -1,7 +1,7 @@
 """A single Swendsen-Wang update on the GPU (mirror of ``src/rbim/swendsen_wang.py``).
 
-``sw_sweep`` runs one sweep of one lattice through the plain engine and
-returns the reference's ``SweepResult``.  It is the per-sweep API; throughput
+``sw_sweep`` runs one sweep of one lattice on the engine ``engine="auto"`` picks
+for it and returns the reference's ``SweepResult``.  It is the per-sweep API; throughput
 work goes through :class:`~.engine.ChainSet` and ``run_temperature_scan``,
 which keep the state on the device across sweeps.
 """
@@ -89,33 +89,26 @@ def sw_sweep(spins: np.ndarray, lattice: Lattice, J: np.ndarray, beta: float, rn
     buffers of L x L lattices are kept between calls (one chain set per device
     and L, used under a lock), so a loop over ``sw_sweep`` allocates device
     memory only on its first call; each call still copies the spins and
-    couplings in and the spins and the record out.
+    couplings in and the spins and the record out, in one copy each way.
     """
     L = lattice.L
     if key is None:
         if rng is None:
             raise ValueError("sw_sweep needs a key or a numpy Generator")
         key = int(rng.integers(0, 2**63, dtype=np.int64))
-    cs, lock, engine = _sweep_chain_set(L, device)
-    with lock:
+    st = _sweep_state(L, device)
+    with st.lock:
         # One chain whose only sweep is `sweep`: measured when n_therm == sweep.
-        cs.coupling_pool[: 2 * words_for(L)].copy_(_torch().from_numpy(pack_couplings(J, L).view(np.int32)))
-        cs.set_spins(0, pack_spins(spins, L))
-        cs.set_descriptor_fields(0, key=int(key) & (2**64 - 1), thr=threshold(beta), sweep=sweep,
-                                 n_therm=sweep if measure else sweep + 1, n_bins=1, sweeps_per_bin=1)
-        cs.acc_int.zero_()
-        cs.acc_f64.zero_()
-        if engine == "grid":
-            cs.run_grid(1)  # one cooperative launch over every SM
-        elif engine == "batched":
-            cs.run_batched(1, threads=single_cta_threads(L))  # one resident CTA
-        else:
-            cs.run_plain(1)
-        cs.check_status()
-        spins[...] = unpack_spins(cs.spin_words(0), L, dtype=spins.dtype)
+        st.couplings[:] = pack_couplings(J, L)
+        st.spins[:] = pack_spins(spins, L)
+        d = st.desc
+        d["key"], d["thr"], d["sweep"] = int(key) & (2**64 - 1), threshold(beta), sweep
+        d["n_therm"] = sweep if measure else sweep + 1
+        st.run()
+        spins[...] = unpack_spins(st.spins, L, dtype=spins.dtype)
         if not measure:
             return None
-        rec = cs.chain_records(0)[0]
+        rec = st.record.copy()
     wx = bool(rec[7]) if measure_percolation else None
     wy = bool(rec[8]) if measure_percolation else None
     return SweepResult(energy=float(rec[0]), magnetization=float(rec[1]), n_clusters=int(rec[2]),
@@ -123,23 +116,70 @@ def sw_sweep(spins: np.ndarray, lattice: Lattice, J: np.ndarray, beta: float, rn
                        second_abs_magnetization=float(rec[6]), wraps_x=wx, wraps_y=wy)
 
 
-_sets_lock = threading.Lock()
-_sets = {}  # (device, L) -> (ChainSet of one chain with a one-row record buffer, its lock, engine)
+class _SweepState:
+    """Device and host buffers of ``sw_sweep`` for L x L lattices on one device, used under ``lock``.
+
+    The chain set's inputs (bin sums, couplings, descriptor, spins) and its
+    outputs (spins, record, status) lie in one device buffer, mirrored in one
+    pinned host buffer, so that a call makes one copy in and one copy out.
+    """
+
+    def __init__(self, L: int, dev):
+        torch = _torch()
+        spec = ChainSpec(L=L, realization=0, key=0, beta=1.0, n_therm=0, n_bins=1, sweeps_per_bin=1, records=True)
+        cs = ChainSet([spec], [np.zeros(2 * words_for(L), dtype="<u4")], device=dev)
+        with torch.cuda.device(dev):
+            self.engine = auto_engine([spec])
+        self.lock = threading.Lock()
+        self.chain_set, self.device, self.threads = cs, dev, single_cta_threads(L)
+        at, end = {}, 0
+        for name in ("acc_int", "acc_f64", "coupling_pool", "chains", "spin_pool", "records", "status"):
+            t = getattr(cs, name)
+            at[name] = (end, end + t.numel() * t.element_size())
+            end = (at[name][1] + 15) & ~15
+        device = torch.zeros(end, dtype=torch.uint8, device=dev)
+        host = torch.zeros(end, dtype=torch.uint8, pin_memory=True)
+        for name, (lo, hi) in at.items():
+            t = getattr(cs, name)
+            setattr(cs, name, device[lo:hi].view(t.dtype).view(t.shape))
+        self._in = (device[: at["spin_pool"][1]], host[: at["spin_pool"][1]])
+        self._out = (device[at["spin_pool"][0]:], host[at["spin_pool"][0]:])
+        h = host.numpy()
+        view = lambda name, dtype: h[slice(*at[name])].view(dtype)  # noqa: E731
+        self.couplings, self.spins = view("coupling_pool", "<u4"), view("spin_pool", "<u4")
+        self.record, self.status = view("records", np.int32), view("status", np.int32)
+        self.desc = view("chains", cs.desc_host.dtype)
+        self.desc[:] = cs.desc_host
+
+    def run(self) -> None:
+        """One sweep of the chain described by the host buffer; its spins, record and status come back there."""
+        cs, stream = self.chain_set, _torch().cuda.current_stream(self.device)
+        try:
+            self._in[0].copy_(self._in[1], non_blocking=True)
+            if self.engine == "grid":
+                cs.run_grid(1)  # one cooperative launch over every SM
+            elif self.engine == "batched":
+                cs.run_batched(1, threads=self.threads)  # one resident CTA
+            else:
+                cs.run_plain(1)
+            self._out[1].copy_(self._out[0], non_blocking=True)
+        finally:
+            stream.synchronize()  # the host buffer is free again, whatever happened
+        if self.status[0]:
+            cs.check_status()
 
 
-def _sweep_chain_set(L: int, device):
-    """The device state ``sw_sweep`` reuses for L x L lattices: one chain set per (device, L), created on first
-    use, so that a caller looping over ``sw_sweep`` does not allocate and free device buffers every sweep, and
-    and the engine the sweep runs on: ``auto_engine``'s choice for one lattice."""
+_states_lock = threading.Lock()
+_states = {}  # (device, L) -> _SweepState
+
+
+def _sweep_state(L: int, device) -> _SweepState:
+    """The state ``sw_sweep`` reuses for L x L lattices: one per (device, L), created on first use, so that a caller
+    looping over ``sw_sweep`` does not allocate and free buffers every sweep."""
     dev = require_cuda(device)
     key = (str(dev), int(L))
-    with _sets_lock:
-        entry = _sets.get(key)
-        if entry is None:
-            spec = ChainSpec(L=L, realization=0, key=0, beta=1.0, n_therm=0, n_bins=1, sweeps_per_bin=1, records=True)
-            cs = ChainSet([spec], [np.zeros(2 * words_for(L), dtype="<u4")], device=dev)
-            with _torch().cuda.device(dev):
-                engine = auto_engine([spec])
-            entry = (cs, threading.Lock(), engine)
-            _sets[key] = entry
-        return entry
+    with _states_lock:
+        state = _states.get(key)
+        if state is None:
+            state = _states[key] = _SweepState(L, dev)
+        return state
