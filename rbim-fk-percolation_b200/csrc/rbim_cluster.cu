@@ -49,7 +49,6 @@ constexpr uint32_t kTileMax = 65536;    // 16-bit tile parents
 constexpr uint32_t kTileHalf = 32768;   // tiles of the 512-thread mode
 constexpr uint32_t kClusterMax = 16;    // non-portable cluster size limit
 constexpr uint32_t kHashMax = 4096;     // node slots per tile (12 bits of a node id)
-constexpr uint32_t kHalfTilesMax = 5;   // most tiles per lattice in the 512-thread mode
 constexpr uint32_t kEmptyKey = 0xFFFFFFFFu;
 constexpr size_t kSmemBudget = 227 * 1024 - 4 * 1024;  // one CTA per SM
 constexpr size_t kSmemPerSm = 228 * 1024;
@@ -121,18 +120,23 @@ bool cluster_layout_fits(const ClusterLayout &ly, uint32_t threads)
 
 ClusterPlan cluster_plan(uint32_t L)
 {
-    // Two 512-thread CTAs per SM hide each other's barrier waits better than
-    // one of 1024 (as in the resident engine), but twice the tiles also mean
-    // twice the boundary bonds and wider cluster barriers: on B200 the
-    // smaller tiles win up to 5 per lattice (L = 300: +10 %, L = 384: +6 %)
-    // and lose at 8 (L = 512) and 16 (L = 724).
-    for (uint32_t C = 2; C <= kHalfTilesMax; ++C) {
-        if (!cluster_tiles_ok(L, C, kTileHalf)) continue;
-        if (cluster_layout_fits(cluster_layout(L, C), 512u)) return {C, 512u};
-        break;
-    }
+    // Few large tiles per lattice (each boundary costs), on as many SMs as
+    // clusters of that size fill: of a B200's 148 SMs, clusters of one CTA per
+    // SM fill 148 (2 CTAs), 135 (3), 132 (4), 130 (5), 132 (6), 105 (7), 120
+    // (8), 135 (9), 110 (10), 77 to 105 (11 to 15) and 112 or 128 (16), so 7
+    // and 8 give way to 9, and 11 to 15 to 16.  Two 512-thread CTAs per SM
+    // hide each other's barrier waits better than one of 1024, while twice the
+    // tiles do not cost more than that.  Measured on B200, cycles a site and
+    // SM: L = 300: 3 x 512 3.84, 2 x 1024 4.21; L = 352: 2 x 1024 3.62, 4 x 512
+    // 3.97; L = 384: 5 x 512 4.17, 3 x 1024 4.45; L = 416: 3 x 1024 4.25, 6 x
+    // 512 4.29; L = 640: 9 x 1024 4.89, 7 5.58; L = 896: 16 x 1024 5.51, 13 6.50.
+    const ClusterPlan order[] = {{3, 512},  {2, 1024}, {5, 512},  {3, 1024}, {4, 1024},
+                                 {5, 1024}, {6, 1024}, {9, 1024}, {10, 1024}, {16, 1024}};
+    for (const ClusterPlan p : order)
+        if (cluster_plan_ok(L, p)) return p;
+    // Sizes whose tiles fit none of these.
     for (uint32_t C = 2; C <= kClusterMax; ++C)
-        if (cluster_tiles_ok(L, C) && cluster_layout_fits(cluster_layout(L, C), 1024u)) return {C, 1024u};
+        if (cluster_plan_ok(L, {C, 1024u})) return {C, 1024u};
     return {0u, 0u};
 }
 
@@ -159,7 +163,7 @@ struct CRed {
     // Rank 0's combined results, read by the other CTAs.
     uint32_t g1, g2, ncl_total;
     // Per chain / per sweep state.
-    int item, wrap, err;
+    int item, wrap, err, others;
     uint32_t front, tile_end;
     Acc acc;
     long long cur_bin;
@@ -511,6 +515,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
         tl.x0 = tl.b / tl.L;
         tl.f = tl.b - tl.x0 * tl.L;
         tl.nwp = (((tl.N + 31u) >> 5) + 3u) & ~3u;
+        tl.inv = tile_inv(tl.L);
         const Ctx x = make_ctx(smem, ly, tl, red);
         const Lat<Word16> &t = x.t;
         const Dist d{cl, x.HK, x.HW, x.hs, x.hs_log2, &red.wrap, &red.err, C * x.hs + 64u};
@@ -743,6 +748,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                 // node marks are no longer needed); with `second` in OH, and
                 // those of the second largest in FLIP.
                 uint32_t *mark = second ? t.OH : t.FLIP;
+                if (tid == 0) red.others = 0;
                 for (uint32_t w = tid; w < t.g.NW; w += NT) {
                     t.FLIP[w] = 0u;
                     if (second) t.OH[w] = 0u;
@@ -751,6 +757,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                 if (tid == 0 && g1 >= tl.b && g1 < tl.b + tl.Tc) {
                     const uint32_t m = g1 - tl.b;
                     atomicOr(mark + (m >> 5), 1u << (m & 31u));
+                    if (m != likely) red.others = 1;
                 }
                 if (second && tid == 0 && g2 >= tl.b && g2 < tl.b + tl.Tc) {
                     const uint32_t m = g2 - tl.b;
@@ -764,6 +771,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                     if (gr == g1) {
                         const uint32_t m = x.HK[k];
                         atomicOr(mark + (m >> 5), 1u << (m & 31u));
+                        if (m != likely) red.others = 1;
                     } else if (second && gr == g2) {
                         const uint32_t m = x.HK[k];
                         atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
@@ -774,8 +782,10 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                 if (!second && ((mark[likely >> 5] >> (likely & 31u)) & 1u)) mc = likely_m;
                 // One lane per word, one test per run piece, from the top: a
                 // piece leader's word holds its tile root (the root's own word
-                // its size).  Pieces of the likely largest are summed above.
-                for (uint32_t w = tid; w < t.g.NW; w += NT) {
+                // its size).  Pieces of the likely largest are summed above;
+                // a tile with no other part of the largest cluster is done
+                // (16 k cycles a pass at L = 512).
+                for (uint32_t w = tid; (second || red.others) && w < t.g.NW; w += NT) {
                     const uint32_t valid = t.g.valid(w), skip = second ? 0u : t.OH[w];
                     const uint32_t roots = t.ROOT[w], sw = t.S[w];
                     uint32_t cut = piece_leaders(t, w, valid) & ~(skip & ((skip << 1) | 1u));

@@ -697,6 +697,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
     tl.x0 = tl.b / tl.L;
     tl.f = tl.b - tl.x0 * tl.L;
     tl.nwp = (((tl.N + 31u) >> 5) + 3u) & ~3u;
+    tl.inv = tile_inv(tl.L);
     const uint32_t cap =
         ch.walk_cap > 0 ? (uint32_t)min((long long)ch.walk_cap, (long long)tl.Tc + 64ll) : tl.Tc + 64u;
     const GTile x = make_gtile(smem, ly, tl, red, cap);

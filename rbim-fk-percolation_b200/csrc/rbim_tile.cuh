@@ -13,13 +13,17 @@ namespace rbim {
 // Geometry of this CTA's tile of the current chain.
 struct Tile {
     uint32_t L, N, C, c, T, b, Tc, tw, x0, f, nwp;
+    uint32_t inv;  // ceil(2^32 / L) while L^3 < 2^32 (its error then stays below a row), or 0 to divide
+    __device__ __forceinline__ uint32_t row(uint32_t n) const { return inv ? __umulhi(n, inv) : n / L; }
 };
+
+__device__ __forceinline__ uint32_t tile_inv(uint32_t L) { return L <= 1625u ? 0xFFFFFFFFu / L + 1u : 0u; }
 
 // Row-end bit of tile word w (at most one: L > 32).
 __device__ __forceinline__ uint32_t tile_row_end(const Tile &tl, uint32_t w, uint32_t valid)
 {
     const uint32_t n0 = tl.b + (w << 5);
-    const uint32_t p = (tl.L - 1u) - (n0 % tl.L);
+    const uint32_t p = (tl.L - 1u) - (n0 - tl.row(n0) * tl.L);
     return p < 32u ? (1u << p) & valid : 0u;
 }
 
@@ -85,7 +89,7 @@ __device__ __forceinline__ void tile_activate(const Lat<Word16> &t, uint32_t *YS
             t.OV[w] = keep;
             if (ov & re) {
                 const uint32_t bit = __ffs(re) - 1u;
-                const uint32_t row = (tl.b + (w << 5) + bit + 1u) / tl.L - 1u - tl.x0;
+                const uint32_t row = tl.row(tl.b + (w << 5) + bit) - tl.x0;
                 atomicOr(YS + (row >> 5), 1u << (row & 31u));
             }
         }
