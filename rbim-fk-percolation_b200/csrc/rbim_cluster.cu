@@ -392,9 +392,14 @@ __device__ __forceinline__ void tile_boundary(const Ctx &x, const Tile &tl, cons
             ra = tile_root_walk(t.uf.w, a, t.cap, d.err);
             rb = (tb << 16) | tile_root_walk(ufb, bl, t.cap, d.err);
         }
-        // A bond joining the same two tile roots with the same seam crossing
-        // as the previous lane's closes a loop of winding zero (paths inside a
-        // tile never wrap) and changes nothing.
+        // A y-seam bond inside one tile cluster closes a loop that winds once
+        // (paths inside a tile never wrap).  A bond joining the same two tile
+        // roots with the same seam crossing as the previous lane's closes a
+        // loop of winding zero and changes nothing.
+        if (live && rb == ((tl.c << 16) | ra)) {
+            atomicOr(d.wrap, 2);
+            live = false;
+        }
         const int tag = live ? 1 + ex + 2 * ey : 0;
         const uint32_t pra = __shfl_up_sync(0xFFFFFFFFu, ra, 1), prb = __shfl_up_sync(0xFFFFFFFFu, rb, 1);
         const int ptag = __shfl_up_sync(0xFFFFFFFFu, tag, 1);

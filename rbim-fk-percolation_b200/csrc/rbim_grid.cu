@@ -558,6 +558,11 @@ __device__ __forceinline__ void grid_boundary(const GTile &x, const Tile &tl, co
                 ey = 1;
             }
         }
+        // A y-seam bond inside one tile cluster closes a loop that winds once.
+        if (live && ra == rb) {
+            atomicOr(d.wrap, 2);
+            live = false;
+        }
         const int tag = live ? 1 + ex + 2 * ey : 0;
         const uint32_t pra = __shfl_up_sync(0xFFFFFFFFu, ra, 1), prb = __shfl_up_sync(0xFFFFFFFFu, rb, 1);
         const int ptag = __shfl_up_sync(0xFFFFFFFFu, tag, 1);

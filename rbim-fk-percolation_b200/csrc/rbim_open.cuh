@@ -455,21 +455,21 @@ __device__ __forceinline__ void roots_flip_sites(const Lat<Word16> &t, uint32_t 
     for (uint32_t w0 = K * warp; w0 < g.NW; w0 += K * nwarps) {
         const uint32_t n0 = (w0 << 5) + lane;
         // Lanes past the lattice walk from site 0, which is a root.  Two steps
-        // a vote.
-        uint32_t r[K];
+        // a vote, the first two without one (hardly any group ends there).
+        uint32_t p[K], r[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) r[k] = uf.ld(n0 + 32u * k < g.N ? n0 + 32u * k : 0u);
         for (uint32_t it = 0;; ++it) {
-            uint32_t p[K];
-            bool moved = false;
 #pragma unroll
             for (int k = 0; k < K; ++k) p[k] = uf.ld(r[k]);
 #pragma unroll
             for (int k = 0; k < K; ++k) r[k] = uf.ld(p[k]);
+            if (it == 0) continue;
+            bool moved = false;
 #pragma unroll
             for (int k = 0; k < K; ++k) moved |= p[k] != r[k];
             if (!__any_sync(0xFFFFFFFFu, moved)) break;
-            if (it >= t.cap) {
+            if (it > t.cap) {
                 if (moved) atomicOr(t.err, kErrFindCap);
                 break;
             }

@@ -43,9 +43,11 @@ __host__ __device__ constexpr size_t align16(size_t v) { return (v + 15) & ~size
 
 __host__ __device__ constexpr uint32_t hash_size(uint32_t l_max)
 {
-    // At most 4L distinct open roots touch a seam bond; keep the load <= 1/2.
+    // A slot for every end of the 2L seam bonds; few of them are ever taken
+    // (bonds inside one open cluster need none, clusters have several ends),
+    // and every slot is reset and looked at in every sweep.
     uint32_t h = 32;
-    while (h < 8u * l_max) h *= 2;
+    while (h < 4u * l_max) h *= 2;
     return h;
 }
 
@@ -137,14 +139,15 @@ __host__ __device__ constexpr ResidentLayout resident_layout_c(uint32_t l_max, i
     ly.off_HW = off;
     off += 4ull * ly.hs;
     // The warps' union lists, in the seam tables' memory (reset after the
-    // unions) where that gives every warp at least 32 entries.
+    // unions) where that gives every warp at least 128 entries, else beside it:
+    // 256 entries in CTAs that have the SM to themselves, 32 in others.
     const uint32_t nwarps = (uint32_t)threads / 32u;
     ly.off_LIST = ly.off_HK;
     ly.seg = 4u * ly.hs / nwarps;
-    if (ly.seg < 32u) {
+    if (ly.seg < 128u || threads == 1024) {
         ly.off_LIST = off;
-        ly.seg = 32u;
-        off += 64ull * nwarps;
+        ly.seg = threads == 1024 ? 256u : 32u;
+        off += 2ull * ly.seg * nwarps;
     }
     ly.bytes = align16(off);
     return ly;
@@ -169,13 +172,13 @@ int resident_default_threads(int l_max)
     // barrier waits better than one large one; so the CTA is as small as the
     // lattice allows before its per-thread work grows long and its shared
     // memory keeps threads off the SM.  Measured on B200, cycles a site and SM
-    // with half / this / twice the threads: L = 32: - / 4.4 / 4.7; L = 40: 5.0
-    // / 4.5 / 5.0; L = 48: 4.4 / 4.2 / 5.0; L = 64: 3.3 / 2.7 / 3.4; L = 72: 3.4
-    // / 3.1 / 4.7; L = 124: 3.2 / 2.3 / 2.8; L = 144: 3.4 / 2.7 / 3.4; L = 181:
-    // 3.2 / 2.4 / 2.7, and above, where one CTA of 512 threads would have the
-    // SM to itself, L = 192: 5.3 / 3.6 / 2.9.
+    // with half / this / twice the threads: L = 32: - / 4.2 / 4.5; L = 40: 5.0
+    // / 4.2 / 5.0; L = 48: - / 4.0 / 4.1; L = 64: 3.0 / 2.7 / 3.3; L = 72: 3.1
+    // / 3.0 / 4.6; L = 124: 3.2 / 2.1 / 2.8; L = 144: 2.6 / 2.6 / 3.3; L = 192:
+    // 3.1 / 2.6 / 2.8, and above, where one CTA of 512 threads would have the
+    // SM to itself, L = 224: 5.4 / 3.4 / 2.6.
     if (l_max <= 32) return 32;
-    if (l_max <= 44) return 64;
+    if (l_max <= 48) return 64;
     if (l_max <= 64) return 128;
     if (l_max <= 128) return 256;
     if (2 * (resident_layout_c((uint32_t)l_max, 512).bytes + kStaticSmem) <= kSmemPerSm) return 512;
@@ -307,32 +310,53 @@ __device__ __forceinline__ void seam_reset(const Res &r, uint32_t warp, uint32_t
 }
 
 // (b) Seam bonds: x seam (x = L-1 -> 0, crossing (1,0)) and y seam
-// (y = L-1 -> 0, crossing (0,1)).  The open union-find is final here.
+// (y = L-1 -> 0, crossing (0,1)).  The open union-find is final here.  A bond
+// inside one open cluster closes a loop that winds once (no path inside the
+// open lattice crosses a seam) and needs no node; one that joins the same two
+// open clusters with the same crossing as the lane before closes a loop of
+// winding zero.
 __device__ __forceinline__ void phase_seam(const Res &r, uint32_t tid, uint32_t nthreads)
 {
     const Lat<Word16> &t = r.t;
     const Geom &g = t.g;
-    for (uint32_t i = tid; i < 2u * g.L; i += nthreads) {
-        uint32_t a, b;
-        int ex, ey;
+    const uint32_t lane = tid & 31u;
+    for (uint32_t i0 = tid & ~31u; i0 < 2u * g.L; i0 += nthreads) {
+        const uint32_t i = i0 + lane;
+        uint32_t a = 0, b = 0;
+        int ex = 0, ey = 0;
         if (i < g.L) {
             a = g.N - g.L + i;
-            if (!((t.OH[a >> 5] >> (a & 31u)) & 1u)) continue;
             b = i;
-            ex = 1;
-            ey = 0;
-        } else {
+            ex = (t.OH[a >> 5] >> (a & 31u)) & 1u;
+        } else if (i < 2u * g.L) {
             const uint32_t x = i - g.L;
-            if (!((t.SEAMV[x >> 5] >> (x & 31u)) & 1u)) continue;
-            a = x * g.L + g.L - 1u;
             b = x * g.L;
-            ex = 0;
-            ey = 1;
+            a = b + g.L - 1u;
+            ey = (t.SEAMV[x >> 5] >> (x & 31u)) & 1u;
         }
-        const uint32_t ra = uf_root_ro<Word16>(t.uf, a, t.cap, t.err);
-        const uint32_t rb = uf_root_ro<Word16>(t.uf, b, t.cap, t.err);
-        const uint32_t na = hash_insert(r, ra, t.err);
-        const uint32_t nb = hash_insert(r, rb, t.err);
+        bool live = ex | ey;
+        if (live) {
+            for (uint32_t it = 0;; ++it) {
+                const uint32_t pa = t.uf.ld(a), pb = t.uf.ld(b);
+                if (pa == a && pb == b) break;
+                a = pa;
+                b = pb;
+                if (it >= t.cap) {
+                    atomicOr(t.err, kErrFindCap);
+                    break;
+                }
+            }
+            if (a == b) {
+                atomicOr(t.wrap, ex | 2 * ey);
+                live = false;
+            }
+        }
+        const uint32_t what = live ? (a << 16 | b) : 0u;  // a != b, so never 0
+        const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, what, 1);
+        const int ex_before = __shfl_up_sync(0xFFFFFFFFu, ex, 1);
+        if (!live || (lane > 0u && before == what && ex_before == ex)) continue;
+        const uint32_t na = hash_insert(r, a, t.err);
+        const uint32_t nb = hash_insert(r, b, t.err);
         seam_union(r, na, nb, ex, ey, t.wrap, t.cap, t.err);
     }
 }
