@@ -31,7 +31,8 @@
 //     barrier at the end of the call), off the critical path of the sweep.
 //
 // Every load of data another CTA wrote during the launch bypasses L1
-// (ld.global.cg): L1 is not coherent across SMs.  Every wait at a grid
+// (ld.global.cg): L1 is not coherent across SMs; only the union-find walks
+// may read words as old as the last grid barrier (GDist).  Every wait at a grid
 // barrier is bounded; a CTA that gives up sets RBIM_STATUS_GRID_WAIT and an
 // abort flag after which no CTA waits again, so the launch always ends.
 #include <algorithm>
@@ -251,8 +252,7 @@ __device__ __forceinline__ void grid_sync(GridSync *gs, uint32_t nblocks, long l
 }
 
 // Union-find over the nodes in global memory: node = global site of a tile
-// root, key = node, words Word64 (parent | wx | wy).  Loads bypass L1 (words
-// change during the launch and from sweep to sweep).  Every node index is
+// root, key = node, words Word64 (parent | wx | wy).  Every node index is
 // checked against the lattice before it is used: after a barrier gave up, a
 // CTA may read node ids another CTA has not written yet (the workspace holds
 // arbitrary bytes), and such an id ends the walk with an error bit instead of
@@ -262,14 +262,23 @@ struct GDist {
     int *wrap, *err;
     uint32_t cap, n_sites;
 
-    __device__ __forceinline__ unsigned long long ld(uint32_t n) const { return __ldcg(G + n); }
+    // Walk loads may be served by the SM's L1, which every grid barrier
+    // invalidates (its acquire): a word then is at most as old as the last
+    // barrier.  Pointers only move to ancestors and a former root never
+    // becomes a root again, so an old word still names an ancestor with the
+    // right image offset, and every hook is a CAS that re-checks the root in
+    // L2; a walk that such a CAS turned down goes on from the words it saw
+    // there.  The words near a large cluster's root are read by every walk:
+    // with loads from L2 one L = 1024 lattice takes 56 us a sweep, 50 this way.
+    __device__ __forceinline__ unsigned long long ldc(uint32_t n) const { return __ldca(G + n); }
     __device__ __forceinline__ void st(uint32_t n, unsigned long long v) const { __stcg(G + n, v); }
 
+    // Root of node n once the unions are over (after the barrier).
     __device__ __forceinline__ uint32_t root_ro(uint32_t n) const
     {
         uint32_t node = n;
         for (uint32_t it = 0;; ++it) {
-            const uint32_t p = Word64::parent(ld(node));
+            const uint32_t p = Word64::parent(ldc(node));
             if (p == node) break;
             if (it >= cap || p >= n_sites) {
                 atomicOr(err, kErrFindCap);
@@ -280,79 +289,81 @@ struct GDist {
         return node;
     }
 
-    // One path-halving step of the walk at x (summed image offset ox, oy):
-    // true when x is a root, false after moving x two levels up.  An id
-    // outside the lattice sets `bad` and stops the walk.
-    __device__ __forceinline__ bool hstep(uint32_t &x, int &ox, int &oy, bool &bad) const
+    // One path-halving step of a walk: true when it stands on a node whose
+    // word says it is a root.  An id outside the lattice sets `bad` and stops
+    // the walk.
+    __device__ __forceinline__ bool step(Walk<Word64> &k, bool &bad) const
     {
-        const unsigned long long w = ld(x);
-        const uint32_t p = Word64::parent(w);
-        if (p == x) return true;
+        const uint32_t p = Word64::parent(k.w);
+        if (p == k.node) return true;
         if (p >= n_sites) {
             bad = true;
             return true;
         }
-        const unsigned long long wp = ld(p);
+        const unsigned long long wp = ldc(p);
         const uint32_t gp = Word64::parent(wp);
         if (gp == p) {
-            ox += Word64::ox(w);
-            oy += Word64::oy(w);
-            x = p;
+            k.ax += Word64::ox(k.w);
+            k.ay += Word64::oy(k.w);
+            k.node = p;
+            k.w = wp;
             return true;
         }
         if (gp >= n_sites) {
             bad = true;
             return true;
         }
-        const int nx = Word64::ox(w) + Word64::ox(wp), ny = Word64::oy(w) + Word64::oy(wp);
-        st(x, Word64::make(gp, nx, ny));
-        ox += nx;
-        oy += ny;
-        x = gp;
+        const int nx = Word64::ox(k.w) + Word64::ox(wp), ny = Word64::oy(k.w) + Word64::oy(wp);
+        st(k.node, Word64::make(gp, nx, ny));
+        k.ax += nx;
+        k.ay += ny;
+        k.node = gp;
+        k.w = ldc(gp);
         return false;
     }
 
-    // Union across a boundary bond a -> b with seam crossing (ex, ey).  Both
+    // Union across a boundary bond na -> nb with seam crossing (ex, ey).  Both
     // endpoint walks advance in the same iteration (their loads overlap);
     // once both are at roots the larger root is hooked under the smaller with
     // a CAS that re-checks it is still a root, and a lost race resumes the
     // walks from where they stand.
-    __device__ __forceinline__ void unite(uint32_t a, uint32_t b, int ex, int ey) const
+    __device__ __forceinline__ void unite(uint32_t na, uint32_t nb, int ex, int ey) const
     {
-        if (a >= n_sites || b >= n_sites) {
+        if (na >= n_sites || nb >= n_sites) {
             atomicOr(err, kErrFindCap);
             return;
         }
-        int axa = 0, aya = 0, axb = 0, ayb = 0;
-        bool da = false, db = false, bad = false;
+        Walk<Word64> a{ldc(na), na, 0, 0}, b{ldc(nb), nb, 0, 0};
         for (uint32_t it = 0; it < cap; ++it) {
-            if (!da) da = hstep(a, axa, aya, bad);
-            if (!db) db = hstep(b, axb, ayb, bad);
+            bool bad = false;
+            const bool da = step(a, bad), db = step(b, bad);
             if (bad) {
                 atomicOr(err, kErrFindCap);
                 return;
             }
             if (!(da && db)) continue;
-            if (a == b) {
+            if (a.node == b.node) {
                 int f = 0;
-                if (Word64::nonzero(ex + axb - axa)) f |= 1;
-                if (Word64::nonzero(ey + ayb - aya)) f |= 2;
+                if (Word64::nonzero(ex + b.ax - a.ax)) f |= 1;
+                if (Word64::nonzero(ey + b.ay - a.ay)) f |= 2;
                 if (f) atomicOr(wrap, f);
                 return;
             }
-            if (a < b) {
-                const unsigned long long expect = Word64::make(b, 0, 0);
-                if (atomicCAS(G + b, expect, Word64::make(a, axa - ex - axb, aya - ey - ayb)) == expect) return;
+            if (a.node < b.node) {
+                const unsigned long long expect = Word64::make(b.node, 0, 0);
+                b.w = atomicCAS(G + b.node, expect, Word64::make(a.node, a.ax - ex - b.ax, a.ay - ey - b.ay));
+                if (b.w == expect) return;
+                a.w = __ldcg(G + a.node);
             } else {
-                const unsigned long long expect = Word64::make(a, 0, 0);
-                if (atomicCAS(G + a, expect, Word64::make(b, axb + ex - axa, ayb + ey - aya)) == expect) return;
+                const unsigned long long expect = Word64::make(a.node, 0, 0);
+                a.w = atomicCAS(G + a.node, expect, Word64::make(b.node, b.ax + ex - a.ax, b.ay + ey - a.ay));
+                if (a.w == expect) return;
+                b.w = __ldcg(G + b.node);
             }
-            da = db = false;
         }
         atomicOr(err, kErrUnionCap);
     }
 };
-
 
 // Shared scratch of one CTA.
 struct GRed {
@@ -573,6 +584,15 @@ __device__ __forceinline__ void grid_boundary(const GTile &x, const Tile &tl, co
             live = bh_insert(x.BH, bh - 1u,
                              ((unsigned long long)(ra - tl.b) << 34) | ((unsigned long long)rb << 2) |
                                  (unsigned long long)(ex + 2 * ey));
+        // The first bond into a node of the next tile hooks it under this
+        // tile's node, without a walk: the tree of a root rb > ra holds only
+        // nodes from rb on, so ra cannot be in it.  (One L = 249 lattice 35.8
+        // -> 34.4 us a sweep; hooking only every other tile, for shallower
+        // trees, 34.6.)
+        if (live && !(ex | ey) && rb > ra && rb < tl.N) {
+            const unsigned long long self = Word64::make(rb, 0, 0);
+            if (atomicCAS(ws.G + rb, self, Word64::make(ra, 0, 0)) == self) live = false;
+        }
         if (live) d.unite(ra, rb, ex, ey);
     }
 }
@@ -1100,18 +1120,22 @@ bool grid_plan_ok(uint32_t L, GridPlan p) { return grid_fit(L, p, nullptr); }
 
 GridPlan grid_plan(uint32_t L)
 {
-    // 1024-thread CTAs, one tile of about 1024 sites each (smaller tiles add
-    // boundary unions, larger ones add walk latency inside the tile), at most
-    // one per SM; then the largest tile count at or below that whose tiles all
-    // hold at least L sites.  Measured on B200, one lattice, us per sweep:
-    // L = 64: 29 with 4-8 tiles, 33 with 32; L = 128: 33 with 16 tiles, 37
-    // with 128; L = 256: 37 with 64 tiles; L = 1024: 60-61 with 128-147.
+    // One tile of about 1024 sites per CTA (smaller tiles add boundary unions,
+    // larger ones add walk latency inside the tile), at most one per SM; then
+    // the largest tile count at or below that whose tiles all hold at least L
+    // sites.  512 threads for tiles of up to 1024 sites, else 1024.  Measured
+    // on B200, one lattice, us per sweep: L = 128: 16 x 512 28.0, 16 x 1024
+    // 29.1, 32 x 512 27.6, 8 x 512 28.7; L = 249: 61 x 512 32.0, 61 x 1024 32.8,
+    // 20 x 512 34.7; L = 512: 128 x 1024 37.7, 128 x 512 38.7, 74 x 1024 39.6;
+    // L = 1024: 128 x 1024 50.5, 128 x 512 55.7, 74 x 1024 57.7.
     const int sms = device_sm_count();
     if (sms <= 0) return {0u, 0u};
     const uint64_t want = ((uint64_t)L * L + 1023u) / 1024u;
     uint32_t C = (uint32_t)std::min<uint64_t>((uint64_t)std::max(sms, 2), std::max<uint64_t>(want, 2u));
     for (; C >= 2u; --C)
-        if (grid_plan_ok(L, {C, 1024u})) return {C, 1024u};
+        for (const uint32_t threads : {512u, 1024u})
+            if ((threads == 1024u || cluster_tile_size(L * L, C) <= 1024u) && grid_plan_ok(L, {C, threads}))
+                return {C, threads};
     return {0u, 0u};
 }
 

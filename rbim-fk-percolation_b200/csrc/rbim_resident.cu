@@ -173,12 +173,12 @@ int resident_default_threads(int l_max)
     // lattice allows before its per-thread work grows long and its shared
     // memory keeps threads off the SM.  Measured on B200, cycles a site and SM
     // with half / this / twice the threads: L = 32: - / 4.2 / 4.5; L = 40: 5.0
-    // / 4.2 / 5.0; L = 48: - / 4.0 / 4.1; L = 64: 3.0 / 2.7 / 3.3; L = 72: 3.1
+    // / 4.2 / 5.0; L = 48: 4.0 / 4.1 / 4.9; L = 64: 3.0 / 2.7 / 3.3; L = 72: 3.1
     // / 3.0 / 4.6; L = 124: 3.2 / 2.1 / 2.8; L = 144: 2.6 / 2.6 / 3.3; L = 192:
     // 3.1 / 2.6 / 2.8, and above, where one CTA of 512 threads would have the
     // SM to itself, L = 224: 5.4 / 3.4 / 2.6.
     if (l_max <= 32) return 32;
-    if (l_max <= 48) return 64;
+    if (l_max <= 44) return 64;
     if (l_max <= 64) return 128;
     if (l_max <= 128) return 256;
     if (2 * (resident_layout_c((uint32_t)l_max, 512).bytes + kStaticSmem) <= kSmemPerSm) return 512;

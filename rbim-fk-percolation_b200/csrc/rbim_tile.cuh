@@ -94,9 +94,10 @@ __device__ __forceinline__ void tile_activate(const Lat<Word16> &t, uint32_t *YS
             }
         }
     }
-    // Flip bits: Philox block q of stream 1 covers global words 4q .. 4q+3.
+    // Flip bits: Philox block q of stream 1 covers global words 4q .. 4q+3; from
+    // the last thread on, whose warps have no bonds to draw in small tiles.
     const uint32_t nblk = (g.NW + 3u) >> 2;
-    for (uint32_t q = tid; q < nblk; q += NT) {
+    for (uint32_t q = NT - 1u - tid; q < nblk; q += NT) {
         const U4 rr = philox_block(rng.key, chunk0 + q, rng.sweep, kStreamFlip);
         const uint32_t w = 4u * q;
         t.FLIP[w] = rr.x;

@@ -28,18 +28,18 @@ __all__ = ["ChainSpec", "ChainSet", "chain_key", "require_cuda", "SINGLE_CTA_MAX
 #: A set of one lattice runs under ``engine="auto"`` on one resident CTA when
 #: L <= SINGLE_CTA_MAX_L, with the CTA size ``single_cta_threads(L)``, and
 #: over the whole GPU above: on the grid engine where it has a plan for L, else
-#: on the plain engine.  Measured on B200, one lattice, us per sweep: L = 32,
-#: one CTA of 512 threads 16.5 (64 threads, the batch default, 32.7); L = 48,
-#: one CTA of 1024 threads 22.8, grid engine 28.6; L = 64, 26.0 against 29.9;
-#: L = 96, 42.9 against 32.2.
-SINGLE_CTA_MAX_L = 64
+#: on the plain engine.  Measured on B200, one lattice, us per sweep, one CTA
+#: against the grid engine: L = 64 19.9 / 23.7, L = 96 24.7 / 26.5, L = 112 27.2 /
+#: 27.9, L = 128 29.0 / 28.0.
+SINGLE_CTA_MAX_L = 112
 
 
 def single_cta_threads(L: int) -> int:
     """CTA size for one lattice alone on the resident engine: the large sizes minimise the time per sweep (the
-    batch default favours many CTAs per SM instead).  Measured on B200: 512 threads up to L = 32 (16.1 us at
-    L = 24 and 16.5 at L = 32, against 17.3 with 1024), 1024 above (22.8 us at L = 48 against 25.9 with 512)."""
-    return 512 if L <= 32 else 1024
+    batch default favours many CTAs per SM instead).  Measured on B200, us per sweep with 512 / 1024 threads:
+    L = 24 16.1 / 16.5 and L = 32 16.5 / 17.3 before the labelling got lighter, L = 72 19.6 / 19.7, L = 96 24.7 /
+    24.7, L = 104 24.8 / 26.7, L = 112 27.2 / 27.8."""
+    return 512 if L <= 32 or L > 96 else 1024
 
 
 _sm_counts = {}
@@ -592,12 +592,12 @@ class ChainSet:
         """Run every chain to the end of its run in chunks of ``chunk`` sweeps.
 
         ``engine="auto"`` (``auto_engine``) runs a set of one lattice with
-        L <= 64 on one resident CTA of ``single_cta_threads(L)`` threads, one
-        larger lattice over the whole GPU -- on the grid engine where it has a
-        plan, else on the plain engine -- and any other set on the batched
-        engines.  On B200 a sweep of one L = 256 lattice takes 38 us
-        on the grid engine, 56 us on the plain engine and 158 us on one
-        resident CTA; L = 1024 66 us, 160 us and 189 us on one 16-CTA cluster.
+        L <= SINGLE_CTA_MAX_L on one resident CTA of ``single_cta_threads(L)``
+        threads, one larger lattice over the whole GPU -- on the grid engine
+        where it has a plan, else on the plain engine -- and any other set on
+        the batched engines.  On B200 a sweep of one L = 256 lattice takes 32 us
+        on the grid engine, 56 us on the plain engine and 75 us on one resident
+        CTA; L = 1024 50 us, 160 us and 115 us on one 16-CTA cluster.
         Results are the same on every engine.
         """
         if engine == "auto":
