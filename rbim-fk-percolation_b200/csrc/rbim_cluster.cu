@@ -458,14 +458,20 @@ __device__ __forceinline__ uint32_t node_root(const Ctx &x, uint32_t k)
 // half carries its root node between the two halves of the propagation).
 __device__ __forceinline__ uint32_t node_key(uint32_t hk) { return hk & 0xFFFFu; }
 
-// The open-tile unions as a separate (non-inlined) function: the cluster
-// kernel keeps more state live across its phases than the resident one, and
-// compiled inline this pointer-chasing loop loses registers to it.
+// Phases as separate (non-inlined) functions where that measured faster on
+// B200 (the kernel keeps much state live across its phases): the size count
+// everywhere (L = 512 3.53 -> 3.47 cycles a site and SM), the heads in the
+// 16-CTA class (L = 1024 4.76 -> 4.67).  The unions are faster inline.
 template <int NT>
-static __device__ __noinline__ void cluster_union(const Lat<Word16> &t, unsigned short *list, uint32_t seg,
-                                                  uint32_t warp)
+static __device__ __noinline__ void cluster_count(const Lat<Word16> &t, const uint32_t *skip, uint32_t warp)
 {
-    phase_union_open<false>(t, list, seg, warp, NT / 32);
+    count_pieces<true>(t, t.uf.w, skip, warp, NT / 32);
+}
+
+template <int NT>
+static __device__ __noinline__ void cluster_heads(const Lat<Word16> &t, uint32_t warp)
+{
+    phase_heads_open<false>(t, warp, NT / 32);
 }
 
 // NT threads per CTA.  LC > 0: the layout is cluster_layout_c(LC, CC), a
@@ -550,13 +556,16 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             tile_activate<NT>(x.t, x.YS, tl, make_rng(ch.key, sweep, ch.thr), gJH, gJV, front, red.tile_end, warp,
                               nwarps, tid);
             __syncthreads();
-            phase_heads_open<false>(t, warp, nwarps);
+            if constexpr (CC == 16)
+                cluster_heads<NT>(t, warp);
+            else
+                phase_heads_open<false>(t, warp, nwarps);
             for (uint32_t k = tid; k < x.hs; k += NT) x.HK[k] = kEmptyKey;
             __syncthreads();
             // The warp's union list lies in its share of the node words, which
             // are reset afterwards.
             const uint32_t share = x.hs / nwarps;
-            cluster_union<NT>(t, (unsigned short *)(x.HW + warp * share), 4u * share, warp);
+            phase_union_open<false>(t, (unsigned short *)(x.HW + warp * share), 4u * share, warp, nwarps);
             for (uint32_t k = warp * share + lane; k < (warp + 1u) * share; k += 32u)
                 x.HW[k] = Word64::make((c << 16) | k, 0, 0);
             __syncthreads();
@@ -617,7 +626,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             // cluster, so no add carries out of its 16 bits (tile_size decodes it).
             // The likely largest tile cluster is counted, and its magnetization
             // summed, by popcounts.
-            count_pieces<true>(t, u16, t.OH, warp, nwarps);
+            cluster_count<NT>(t, t.OH, warp);
             int likely_m = 0;
             {
                 uint32_t in = 0;

@@ -598,16 +598,6 @@ __device__ __forceinline__ void grid_boundary(const GTile &x, const Tile &tl, co
 }
 
 
-// The open-tile unions as a separate (non-inlined) function, as in the cluster
-// engine: inline, this pointer-chasing loop loses registers to the state the
-// kernel keeps live across its phases.
-template <int NT>
-static __device__ __noinline__ void grid_union(const Lat<Word16> &t, unsigned short *list, uint32_t seg,
-                                               uint32_t warp)
-{
-    phase_union_open<true>(t, list, seg, warp, NT / 32);
-}
-
 struct GridArgs {
     rbim_chain_t *chain;
     uint32_t *spin_pool;
@@ -769,7 +759,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
         __syncthreads();
         RBIM_GRID_MARK(1);
         const uint32_t seg = ly.list / nwarps;  // union lists, in the node lists' memory
-        grid_union<NT>(t, (unsigned short *)x.NK + warp * seg, seg, warp);
+        phase_union_open<true>(t, (unsigned short *)x.NK + warp * seg, seg, warp, nwarps);
         __syncthreads();
         RBIM_GRID_MARK(2);
         // Every site's word at its tile root, and the ROOT plane.

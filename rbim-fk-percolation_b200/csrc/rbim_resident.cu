@@ -373,6 +373,24 @@ __device__ __forceinline__ void phase_seam_propagate(const Res &r, uint32_t tid,
     }
 }
 
+// Phases as separate (non-inlined) functions, for the CTA sizes where that
+// measured faster on B200 (fewer registers live across the phase than inline;
+// the larger CTAs lose up to 15 % by it).  us a sweep of 16384 lattices,
+// inline against separate: measurement in one-warp CTAs, L = 32: 222 / 203;
+// heads with 64 threads, L = 40: 371 / 354; heads and roots with 128 threads,
+// L = 64: 597 / 576.
+template <int NT, bool kFew>
+static __device__ __noinline__ void separate_heads(const Lat<Word16> &t, uint32_t warp)
+{
+    phase_heads_open<kFew>(t, warp, NT / 32);
+}
+
+template <int NT, bool kSweep, int K>
+static __device__ __noinline__ void separate_roots(const Lat<Word16> &t, uint32_t *in, uint32_t root, uint32_t warp)
+{
+    roots_flip_sites<kSweep, K>(t, in, root, warp, NT / 32);
+}
+
 // The labelling stages shared by the sweep and label kernels, from occupied
 // bond planes to final roots (every site's word at its root, the ROOT plane);
 // barriers between stages.  kSweep: the clusters are flipped, and in measured
@@ -389,7 +407,10 @@ __device__ __forceinline__ uint32_t resident_label(const Res &r, bool measure)
     // warp, many CTAs hide each other's latency) 5.70 / 5.92 / 6.12 / 6.26.
     constexpr int kWords = NT <= 64 ? 1 : 4;
     unsigned short *list = r.LIST + warp * r.seg;
-    phase_heads_open<kFew>(r.t, warp, nwarps);
+    if constexpr (NT == 64 || NT == 128)
+        separate_heads<NT, kFew>(r.t, warp);
+    else
+        phase_heads_open<kFew>(r.t, warp, nwarps);
     __syncthreads();
     RBIM_PHASE_MARK(1);
     phase_union_open<kFew>(r.t, list, r.seg, warp, nwarps);
@@ -404,7 +425,11 @@ __device__ __forceinline__ uint32_t resident_label(const Res &r, bool measure)
     __syncthreads();
     RBIM_PHASE_MARK(4);
     const uint32_t likely = kSweep && measure ? likely_largest(r.t) : 0u;
-    roots_flip_sites<kSweep, kWords>(r.t, kSweep && measure ? r.t.OH : nullptr, likely, warp, nwarps);
+    uint32_t *members = kSweep && measure ? r.t.OH : nullptr;
+    if constexpr (NT == 128)
+        separate_roots<NT, kSweep, kWords>(r.t, members, likely, warp);
+    else
+        roots_flip_sites<kSweep, kWords>(r.t, members, likely, warp, nwarps);
     __syncthreads();
     RBIM_PHASE_MARK(5);
     return likely;
@@ -539,6 +564,13 @@ __device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, u
     __syncthreads();
 }
 
+template <int NT>
+static __device__ __noinline__ void separate_measure(const Res &res, Red<NT> &red, uint32_t likely,
+                                                     long long rec[kRecLen], bool second)
+{
+    resident_measure<NT>(res, red, likely, rec, second);
+}
+
 // LC > 0: the launch's layout is resident_layout_c(LC, NT), a compile-time
 // constant; LC == 0: the layout passed in.
 template <int NT, int LC>
@@ -608,7 +640,10 @@ __global__ void __launch_bounds__(NT, MinBlocks<NT>::value)
             if (measure) {
                 long long rec[kRecLen];
                 const bool want_rec = records && ch.rec_off >= 0;
-                resident_measure<NT>(res, red, likely, rec, want_rec);
+                if constexpr (NT == 32)
+                    separate_measure<NT>(res, red, likely, rec, want_rec);
+                else
+                    resident_measure<NT>(res, red, likely, rec, want_rec);
                 if (tid == 0) {
                     const long long idx = (long long)(sweep - (uint64_t)ch.n_therm);
                     const long long bin = idx / ch.sweeps_per_bin;
