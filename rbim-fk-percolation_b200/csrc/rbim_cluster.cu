@@ -9,8 +9,8 @@
 //     last L sites and the y-bond of the tile's last site reach the next
 //     tile; the spins they need are a halo copied from the neighbour CTA's
 //     shared memory through distributed shared memory);
-//  2. the open-tile labelling of the resident engine (16-bit parents, run
-//     heads, flat union and root walks): inside a tile every cycle is
+//  2. the open-tile labelling of the resident engine (16-bit parents, linked
+//     run heads, unions from per-warp lists): inside a tile every cycle is
 //     contractible;
 //  3. the boundary bonds -- x-bonds from the last L sites of a tile (into the
 //     next tile, or across the x seam from the last tile to the first), the
@@ -159,11 +159,13 @@ struct CRed {
     // This CTA's partial results, read by rank 0 through DSMEM.
     unsigned long long p_k1, p_k2;
     uint32_t p_unsat, p_downs, p_ncl;
-    int p_wrap, p_mc, p_mc2;
+    int p_wrap, p_mc, p_mc2, p_known;
     // Rank 0's combined results, read by the other CTAs.
     uint32_t g1, g2, ncl_total;
+    int pass;
     // Per chain / per sweep state.
-    int item, wrap, err, others;
+    int item, wrap, err;
+    uint32_t likely_downs;
     uint32_t front, tile_end;
     Acc acc;
     long long cur_bin;
@@ -447,31 +449,148 @@ __device__ __forceinline__ void tile_halo(const Ctx &x, const Tile &tl, const cg
 }
 
 
-// Root node of this tile's node in slot k, once the boundary stage is over
-// (the low word of HW; the high word accumulates merged sizes).
+// A node's word once the boundary stage is over: its root node in 16 bits
+// (tile << 12 | slot), and in a root node's word, summed over the nodes of the
+// merged cluster, its down spins (24 bits) and sites (24 bits, at most 2^20).
+__device__ __forceinline__ uint32_t node_pack(uint32_t node) { return (node >> 16) << 12 | (node & 0xFFFu); }
 __device__ __forceinline__ uint32_t node_root(const Ctx &x, uint32_t k)
 {
-    return *((volatile uint32_t *)(x.HW + k));
+    const uint32_t v = *((volatile uint32_t *)(x.HW + k)) & 0xFFFFu;
+    return (v >> 12) << 16 | (v & 0xFFFu);
+}
+__device__ __forceinline__ uint32_t node_downs(unsigned long long w) { return (uint32_t)(w >> 16) & 0xFFFFFFu; }
+__device__ __forceinline__ uint32_t node_size(unsigned long long w) { return (uint32_t)(w >> 40); }
+
+// Slot of the node of tile root m, which is in the table: every slot its probe
+// passes before is taken, so the first whose key's low half is m is its own.
+__device__ __forceinline__ uint32_t node_slot(const Ctx &x, uint32_t m)
+{
+    uint32_t h = (m * 0x9E3779B1u) >> (32u - x.hs_log2);
+    for (uint32_t it = 0; it < x.hs && (x.HK[h] & 0xFFFFu) != m; ++it) h = (h + 1u) & (x.hs - 1u);
+    return h;
 }
 
 // Tile root of the node in slot k: the low half of its hash word (the high
-// half carries its root node between the two halves of the propagation).
+// half carries its root node between the two halves of the propagation, and
+// the tile cluster's down spins during the measurement).
 __device__ __forceinline__ uint32_t node_key(uint32_t hk) { return hk & 0xFFFFu; }
 
 // Phases as separate (non-inlined) functions where that measured faster on
 // B200 (the kernel keeps much state live across its phases): the size count
 // everywhere (L = 512 3.53 -> 3.47 cycles a site and SM), the heads in the
 // 16-CTA class (L = 1024 4.76 -> 4.67).  The unions are faster inline.
+//
+// The size count: sizes minus one onto the tile roots' own indexes (see
+// count_pieces), one lane per word, one add per run piece outside `skip`; for
+// the pieces of nodes (the FLIP plane marks their tile roots) also the down
+// spins, into the node's hash word.
 template <int NT>
-static __device__ __noinline__ void cluster_count(const Lat<Word16> &t, const uint32_t *skip, uint32_t warp)
+static __device__ __noinline__ void cluster_count(const Ctx &x, uint32_t tid)
 {
-    count_pieces<true>(t, t.uf.w, skip, warp, NT / 32);
+    const Lat<Word16> &t = x.t;
+    unsigned short *u16 = t.uf.w;
+    for (uint32_t w = tid; w < t.g.NW; w += NT) {
+        const uint32_t valid = t.g.valid(w), skip = t.OH[w], roots = t.ROOT[w], s = t.S[w];
+        uint32_t cut = piece_leaders(t, w, valid) & ~(skip & ((skip << 1) | 1u));
+        uint32_t left = valid;  // the bits below the last piece
+        while (cut) {
+            const uint32_t b = 31u - __clz(cut), bit = 1u << b;
+            const uint32_t pm = left & (0u - bit);
+            cut ^= bit;
+            left ^= pm;
+            if (skip & bit) continue;
+            const uint32_t n = (w << 5) + b;
+            const bool is_root = roots & bit;
+            const uint32_t r = is_root ? n : (uint32_t)u16[n];
+            add16(u16, r, __popc(pm) - (is_root ? 1u : 0u));
+            if (((t.FLIP[r >> 5] >> (r & 31u)) & 1u) && (pm & s))
+                atomicAdd(x.HK + node_slot(x, r), (uint32_t)__popc(pm & s) << 16);
+        }
+    }
 }
 
 template <int NT>
 static __device__ __noinline__ void cluster_heads(const Lat<Word16> &t, uint32_t warp)
 {
     phase_heads_open<false>(t, warp, NT / 32);
+}
+
+// The magnetizations of this tile's parts of the largest and (second) the
+// second largest cluster, by a pass over the sites: with records, or when the
+// largest cluster lies inside one tile and is not its likely largest.
+template <int NT>
+static __device__ __forceinline__ void cluster_mc_pass(const Ctx &x, const Tile &tl, const cg::cluster_group &cl,
+                                                    CRed &red, bool second, uint32_t tid)
+{
+    const Lat<Word16> &t = x.t;
+    const unsigned short *u16 = t.uf.w;
+    const uint32_t lane = tid & 31u, warp = tid >> 5, g1 = red.g1, g2 = red.g2;
+    constexpr uint32_t nwarps = NT / 32;
+    // Tile roots of the largest cluster, marked in OH, and those
+    // of the second largest in FLIP (whose node marks are no longer
+    // needed).
+    for (uint32_t w = tid; w < t.g.NW; w += NT) {
+        t.OH[w] = 0u;
+        t.FLIP[w] = 0u;
+    }
+    __syncthreads();
+    if (tid == 0 && g1 >= tl.b && g1 < tl.b + tl.Tc) {
+        const uint32_t m = g1 - tl.b;
+        atomicOr(t.OH + (m >> 5), 1u << (m & 31u));
+    }
+    if (second && tid == 0 && g2 >= tl.b && g2 < tl.b + tl.Tc) {
+        const uint32_t m = g2 - tl.b;
+        atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
+    }
+    for (uint32_t k = tid; k < x.hs; k += NT) {
+        if (x.HK[k] == kEmptyKey) continue;
+        const uint32_t r = node_root(x, k), m = node_key(x.HK[k]);
+        const uint32_t rt = r >> 16;
+        const uint32_t gr = rt * tl.T + node_key(*cl.map_shared_rank(x.HK + (r & 0xFFFFu), rt));
+        if (gr == g1)
+            atomicOr(t.OH + (m >> 5), 1u << (m & 31u));
+        else if (second && gr == g2)
+            atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
+    }
+    __syncthreads();
+    int mc = 0, mc2 = 0;
+    // One lane per word, one test per run piece, from the top: a
+    // piece leader's word holds its tile root (the root's own word
+    // its size).
+    for (uint32_t w = tid; w < t.g.NW; w += NT) {
+        const uint32_t roots = t.ROOT[w], sw = t.S[w];
+        uint32_t left = t.g.valid(w);  // the bits below the last piece
+        uint32_t cut = piece_leaders(t, w, left);
+        while (cut) {
+            const uint32_t b = 31u - __clz(cut), bit = 1u << b;
+            const uint32_t pm = left & (0u - bit);
+            cut ^= bit;
+            left ^= pm;
+            const uint32_t n = (w << 5) + b;
+            const uint32_t r = roots & bit ? n : (uint32_t)u16[n];
+            const int m = (int)__popc(pm) - 2 * (int)__popc(pm & sw);
+            if ((t.OH[r >> 5] >> (r & 31u)) & 1u) mc += m;
+            if (second && ((t.FLIP[r >> 5] >> (r & 31u)) & 1u)) mc2 += m;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        mc += __shfl_xor_sync(0xFFFFFFFFu, mc, o);
+        mc2 += __shfl_xor_sync(0xFFFFFFFFu, mc2, o);
+    }
+    if (lane == 0) {
+        red.mcw[warp] = mc;
+        red.mcw2[warp] = mc2;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int s = 0, s2 = 0;
+        for (uint32_t i = 0; i < nwarps; ++i) {
+            s += red.mcw[i];
+            s2 += red.mcw2[i];
+        }
+        red.p_mc = s;
+        red.p_mc2 = s2;
+    }
 }
 
 // NT threads per CTA.  LC > 0: the layout is cluster_layout_c(LC, CC), a
@@ -593,7 +712,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                 if (hk == kEmptyKey) continue;
                 const uint32_t r = ((hk >> 28) << 16) | ((hk >> 16) & 0xFFFu), m = node_key(hk);
                 x.HK[k] = m;
-                x.HW[k] = (unsigned long long)r;
+                x.HW[k] = (unsigned long long)node_pack(r);
                 if (r != ((c << 16) | k)) {
                     const uint32_t mr = node_key(*cl.map_shared_rank(x.HK + (r & 0xFFFFu), r >> 16));
                     const uint32_t *fl = cl.map_shared_rank(t.FLIP, r >> 16);
@@ -612,50 +731,58 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             __syncthreads();
             cl.sync();  // every flip is done
             tile_halo<NT>(x, tl, cl, red, tid);
+            if (measure) {
+                // FLIP (no longer needed this sweep) becomes the plane of
+                // node marks; OV still gives the run pieces.
+                for (uint32_t w = tid; w < t.g.NW; w += NT) t.FLIP[w] = 0u;
+                if (tid == 0) red.likely_downs = 0u;
+            }
             __syncthreads();
 
             if (!measure) continue;
 
             // ---- measurement (reference sw_sweep, src/rbim/swendsen_wang.py:146-172)
             unsigned short *u16 = t.uf.w;
+            for (uint32_t k = tid; k < x.hs; k += NT) {
+                const uint32_t m = x.HK[k];
+                if (m != kEmptyKey) atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
+            }
             uint32_t unsat = 0, downs = 0;
             tile_energy<NT>(x.t, tl, gJH, gJV, red.front, tid, unsat, downs);
+            __syncthreads();
             // Tile cluster sizes minus one added onto each tile root's own index
             // (a root points at itself): afterwards the word of root m reads
             // m + size - 1, below 65536 because m is the smallest site of its tile
             // cluster, so no add carries out of its 16 bits (tile_size decodes it).
-            // The likely largest tile cluster is counted, and its magnetization
-            // summed, by popcounts.
-            cluster_count<NT>(t, t.OH, warp);
-            int likely_m = 0;
+            // The likely largest tile cluster is counted by popcounts.
+            cluster_count<NT>(x, tid);
             {
-                uint32_t in = 0;
+                uint32_t in = 0, in_downs = 0;
                 for (uint32_t w = tid; w < t.g.NW; w += NT) {
                     const uint32_t m = t.OH[w];
                     in += __popc(m) - (w == likely >> 5 ? 1u : 0u);
-                    likely_m += (int)__popc(m) - 2 * (int)__popc(m & t.S[w]);
+                    in_downs += __popc(m & t.S[w]);
                 }
                 in = __reduce_add_sync(0xFFFFFFFFu, in);
+                in_downs = __reduce_add_sync(0xFFFFFFFFu, in_downs);
                 if (lane == 0 && in) add16(u16, likely, in);
+                if (lane == 0 && in_downs) atomicAdd(&red.likely_downs, in_downs);
             }
             __syncthreads();
-            // FLIP (no longer needed this sweep) becomes the plane of node
-            // marks; OV still gives the run pieces of the |M_C| pass.
-            for (uint32_t w = tid; w < t.g.NW; w += NT) t.FLIP[w] = 0u;
-            __syncthreads();
-            // Merged sizes into the root nodes; mark this tile's nodes in FLIP.
-            uint32_t rootnodes = 0;
+            // Merged sizes and down spins into the root nodes.  With the down
+            // spins summed here, |M_C1| needs no second pass over the run
+            // pieces (bound by the integer pipe like the first): B200, cycles
+            // a site and SM, L = 512 3.47 -> 3.44, L = 1024 4.67 -> 4.60.
+            uint32_t nloc = 0;
             for (uint32_t k = tid; k < x.hs; k += NT) {
-                const uint32_t m = x.HK[k];
-                if (m == kEmptyKey) continue;
-                const uint32_t r = node_root(x, k);
-                atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
-                unsigned int *hi = (unsigned int *)(cl.map_shared_rank(x.HW, r >> 16) + (r & 0xFFFFu)) + 1;
-                atomicAdd(hi, tile_size(u16, m));
-                if (r == ((c << 16) | k)) ++rootnodes;
+                const uint32_t hk = x.HK[k];
+                if (hk == kEmptyKey) continue;
+                const uint32_t m = node_key(hk), r = node_root(x, k);
+                const unsigned long long add = (unsigned long long)tile_size(u16, m) << 40 |
+                                               (unsigned long long)(m == likely ? red.likely_downs : hk >> 16) << 16;
+                atomicAdd(cl.map_shared_rank(x.HW, r >> 16) + (r & 0xFFFFu), add);
+                if (r == ((c << 16) | k)) ++nloc;
             }
-            __syncthreads();
-            uint32_t nloc = rootnodes;
             for (uint32_t w = tid; w < t.g.NW; w += NT) nloc += __popc(t.ROOT[w] & ~t.FLIP[w]);
             cl.sync();  // merged sizes are complete
 
@@ -672,7 +799,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             }
             for (uint32_t k = tid; k < x.hs; k += NT) {
                 if (x.HK[k] == kEmptyKey || node_root(x, k) != ((c << 16) | k)) continue;
-                top2_merge(k1, k2, size_key((uint32_t)(x.HW[k] >> 32), tl.b + x.HK[k]), 0ull);
+                top2_merge(k1, k2, size_key(node_size(x.HW[k]), tl.b + node_key(x.HK[k])), 0ull);
             }
             warp_top2(k1, k2);
             uint32_t u = unsat, dn = downs, nc = nloc;
@@ -707,18 +834,37 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                     red.p_downs = sd;
                     red.p_ncl = sn;
                     red.p_wrap = red.wrap;
+                    // The magnetization of the tile's best: summed with the
+                    // sizes for merged clusters, by popcounts for the likely
+                    // largest tile cluster, unknown for any other.
+                    const uint32_t m = 0xFFFFFFFFu - (uint32_t)(a1 & 0xFFFFFFFFull) - tl.b;
+                    red.p_known = 0;
+                    if (a1 && ((t.FLIP[m >> 5] >> (m & 31u)) & 1u)) {
+                        const unsigned long long w = x.HW[node_slot(x, m)];
+                        red.p_mc = (int)node_size(w) - 2 * (int)node_downs(w);
+                        red.p_known = 1;
+                    } else if (a1 && m == likely) {
+                        red.p_mc = (int)tile_size(u16, m) - 2 * (int)red.likely_downs;
+                        red.p_known = 1;
+                    }
                 }
             }
             cl.sync();  // partials are visible
             long long *rec = red.rec;  // rank 0's record of the sweep
+            // |M_C2| only when the chain's records are written (the bin sums
+            // do not use it).
+            const bool second = records && ch.rec_off >= 0;
             if (c == 0 && warp == 0) {
-                unsigned long long a1 = 0, a2 = 0;
+                unsigned long long a1 = 0, a2 = 0, own = 0;
+                int mc = 0, known = 0;
                 uint32_t su = 0, sd = 0, sn = 0;
                 int wr = 0;
                 if (lane < C) {
                     const CRed *o = cl.map_shared_rank(&red, lane);
-                    a1 = o->p_k1;
+                    a1 = own = o->p_k1;
                     a2 = o->p_k2;
+                    mc = o->p_mc;
+                    known = o->p_known;
                     su = o->p_unsat;
                     sd = o->p_downs;
                     sn = o->p_ncl;
@@ -731,10 +877,17 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                     sn += __shfl_xor_sync(0xFFFFFFFFu, sn, o);
                     wr |= __shfl_xor_sync(0xFFFFFFFFu, wr, o);
                 }
+                // The tile whose best is the largest cluster (keys are unique).
+                const uint32_t owner = __ffs(__ballot_sync(0xFFFFFFFFu, own == a1)) - 1u;
+                mc = __shfl_sync(0xFFFFFFFFu, mc, owner);
+                known = __shfl_sync(0xFFFFFFFFu, known, owner);
                 if (lane == 0) {
                     red.g1 = 0xFFFFFFFFu - (uint32_t)(a1 & 0xFFFFFFFFull);
                     red.g2 = 0xFFFFFFFFu - (uint32_t)(a2 & 0xFFFFFFFFull);
                     red.ncl_total = sn;
+                    red.pass = sn > 1u && (second || !known);
+                    rec[4] = mc;
+                    rec[6] = 0;
                     rec[0] = 2ll * (long long)su - 2ll * (long long)tl.N;
                     rec[1] = (long long)tl.N - 2ll * (long long)sd;
                     rec[2] = sn;
@@ -750,96 +903,15 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                 red.g1 = o->g1;
                 red.g2 = o->g2;
                 red.ncl_total = o->ncl_total;
+                red.pass = o->pass;
             }
             __syncthreads();
-            const uint32_t g1 = red.g1, g2 = red.g2;
-            const bool many = red.ncl_total > 1u;
-            // |M_C2| only when the chain's records are written (the bin sums
-            // do not use it).
-            const bool second = records && ch.rec_off >= 0;
-            if (many) {
-                // Tile roots of the largest cluster, marked in FLIP (whose
-                // node marks are no longer needed); with `second` in OH, and
-                // those of the second largest in FLIP.
-                uint32_t *mark = second ? t.OH : t.FLIP;
-                if (tid == 0) red.others = 0;
-                for (uint32_t w = tid; w < t.g.NW; w += NT) {
-                    t.FLIP[w] = 0u;
-                    if (second) t.OH[w] = 0u;
-                }
-                __syncthreads();
-                if (tid == 0 && g1 >= tl.b && g1 < tl.b + tl.Tc) {
-                    const uint32_t m = g1 - tl.b;
-                    atomicOr(mark + (m >> 5), 1u << (m & 31u));
-                    if (m != likely) red.others = 1;
-                }
-                if (second && tid == 0 && g2 >= tl.b && g2 < tl.b + tl.Tc) {
-                    const uint32_t m = g2 - tl.b;
-                    atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
-                }
-                for (uint32_t k = tid; k < x.hs; k += NT) {
-                    if (x.HK[k] == kEmptyKey) continue;
-                    const uint32_t r = node_root(x, k);
-                    const uint32_t rt = r >> 16;
-                    const uint32_t gr = rt * tl.T + *cl.map_shared_rank(x.HK + (r & 0xFFFFu), rt);
-                    if (gr == g1) {
-                        const uint32_t m = x.HK[k];
-                        atomicOr(mark + (m >> 5), 1u << (m & 31u));
-                        if (m != likely) red.others = 1;
-                    } else if (second && gr == g2) {
-                        const uint32_t m = x.HK[k];
-                        atomicOr(t.FLIP + (m >> 5), 1u << (m & 31u));
-                    }
-                }
-                __syncthreads();
-                int mc = 0, mc2 = 0;
-                if (!second && ((mark[likely >> 5] >> (likely & 31u)) & 1u)) mc = likely_m;
-                // One lane per word, one test per run piece, from the top: a
-                // piece leader's word holds its tile root (the root's own word
-                // its size).  Pieces of the likely largest are summed above;
-                // a tile with no other part of the largest cluster is done
-                // (16 k cycles a pass at L = 512).
-                for (uint32_t w = tid; (second || red.others) && w < t.g.NW; w += NT) {
-                    const uint32_t valid = t.g.valid(w), skip = second ? 0u : t.OH[w];
-                    const uint32_t roots = t.ROOT[w], sw = t.S[w];
-                    uint32_t cut = piece_leaders(t, w, valid) & ~(skip & ((skip << 1) | 1u));
-                    uint32_t left = valid;  // the bits below the last piece
-                    while (cut) {
-                        const uint32_t b = 31u - __clz(cut), bit = 1u << b;
-                        const uint32_t pm = left & (0u - bit);
-                        cut ^= bit;
-                        left ^= pm;
-                        if (skip & bit) continue;
-                        const uint32_t n = (w << 5) + b;
-                        const uint32_t r = roots & bit ? n : (uint32_t)u16[n];
-                        const int m = (int)__popc(pm) - 2 * (int)__popc(pm & sw);
-                        if ((mark[r >> 5] >> (r & 31u)) & 1u) mc += m;
-                        if (second && ((t.FLIP[r >> 5] >> (r & 31u)) & 1u)) mc2 += m;
-                    }
-                }
-                for (int o = 16; o > 0; o >>= 1) {
-                    mc += __shfl_xor_sync(0xFFFFFFFFu, mc, o);
-                    mc2 += __shfl_xor_sync(0xFFFFFFFFu, mc2, o);
-                }
-                if (lane == 0) {
-                    red.mcw[warp] = mc;
-                    red.mcw2[warp] = mc2;
-                }
-                __syncthreads();
-                if (tid == 0) {
-                    int s = 0, s2 = 0;
-                    for (uint32_t i = 0; i < nwarps; ++i) {
-                        s += red.mcw[i];
-                        s2 += red.mcw2[i];
-                    }
-                    red.p_mc = s;
-                    red.p_mc2 = s2;
-                }
-            }
-            cl.sync();  // M_C partials are visible
+            const bool pass = red.pass;
+            if (pass) cluster_mc_pass<NT>(x, tl, cl, red, second, tid);
+            if (pass) cl.sync();  // M_C partials are visible (the same on every CTA)
             if (c == 0 && tid == 0) {
-                long long mc_total = rec[1], mc2_total = 0;
-                if (many) {
+                long long mc_total = red.ncl_total > 1u ? rec[4] : rec[1], mc2_total = 0;
+                if (pass) {
                     mc_total = 0;
                     for (uint32_t i = 0; i < C; ++i) {
                         const CRed *o = cl.map_shared_rank(&red, i);

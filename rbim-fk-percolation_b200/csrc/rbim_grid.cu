@@ -9,8 +9,8 @@
 //  1. activation of the bonds owned by the tile's sites (the spins of the
 //     next tile's first row, and the row start of a partial first row, come
 //     from the global spin plane, which every tile rewrites after its flip);
-//  2. the open-tile labelling of the resident engine (16-bit parents, run
-//     heads, flat union and root walks);
+//  2. the open-tile labelling of the resident engine (16-bit parents, linked
+//     run heads, unions from per-warp lists);
 //  3. the tile roots that boundary bonds can touch become nodes of a
 //     union-find in global memory, one Word64 per site (parent | wx | wy),
 //     indexed by global site; after a grid barrier the boundary bonds --
@@ -22,7 +22,7 @@
 //     around the torus (src/rbim/_unionfind.py:104-124);
 //  4. after a second barrier every node finds its root and takes the root's
 //     raw flip bit (published before the first barrier); the tile flips by
-//     run pieces and writes its spins back (measured sweeps also add their
+//     sites and writes its spins back (measured sweeps also add their
 //     cluster sizes into the root nodes' words); a third barrier;
 //  5. measured sweeps: every CTA's partials (top two, energy, magnetization,
 //     clusters, wraps) are combined by every CTA after a fourth barrier, the
