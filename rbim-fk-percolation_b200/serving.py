@@ -392,7 +392,7 @@ class ScanServer:
                     nt = self.threads or autotune.tuned_threads(l_max, self.device)
                     if not nt:
                         nt = occupancy_threads(int(self.lib.rbim_resident_threads(l_max)), count,
-                                               _sm_count(self.device))
+                                               _sm_count(self.device), l_max * l_max)
                     on_chip.append(Launch(0, base, count, l_max, nt))
                 elif key[0] == 1:
                     plan = autotune.tuned_cluster_plan(l_max, sorted({a.plan.L for a in group}), self.device)

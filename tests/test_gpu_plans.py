@@ -1,4 +1,5 @@
-"""Default cluster plans at the edges of their ranges, with and without per-sweep records.
+"""Default launch plans: cluster plans at the edges of their ranges, with and without per-sweep records, and the CTA
+sizes of launches of few lattices.
 
 The magnetization of the largest cluster is summed with the merged sizes, or by popcounts when it is a tile's likely
 largest cluster, or by a pass over the sites: with records, and when it lies inside one tile without being that
@@ -35,3 +36,29 @@ def test_cluster_plan_edges_match_oracle(rb, orc, L):
             gi, _ = cs.bins(k)
             assert np.array_equal(gi, ib), (L, hot, s)
             assert np.array_equal(cs.spins(k), spins.astype(np.int64)), (L, hot, s)
+
+
+@pytest.mark.parametrize("n", [2, 149, 300, 600, 1300])
+def test_few_lattice_cta_sizes_match_oracle(rb, orc, n):
+    """The CTA size of a launch of few lattices: never above the occupancy bound, a supported size from the
+    library's default on, and the same chains whatever it is."""
+    occ = rb.engine.occupancy_threads
+    for L in range(3, 200):
+        d = rb._native.lib().rbim_resident_threads(L)
+        t = occ(d, n, 148, L * L)
+        assert d <= t <= occ(d, n, 148) and t in (32, 64, 128, 256, 512, 1024), (L, n)
+    for L in (7, 16, 32, 45, 96):
+        J = np.where(np.random.default_rng(L).random(2 * L * L) < 0.1, -1, 1).astype(np.int8)
+        specs = [rb.ChainSpec(L=L, realization=0, key=31 * L + i, beta=1.0 / (0.8 + 0.3 * (i % 8)), n_therm=1, n_bins=2,
+                              sweeps_per_bin=2) for i in range(n)]
+        cs = rb.ChainSet(specs, [rb.packing.pack_couplings(J, L)])
+        cs.init_spins(hot=True)
+        cs.run_batched(5)
+        cs.check_status()
+        for i in sorted({0, 1, n // 2, n - 2, n - 1}):
+            s = specs[i]
+            ib, _, spins = orc.run_chain(L, J, s.key, rb.packing.threshold(s.beta), hot=True, n_therm=1, n_bins=2,
+                                         sweeps_per_bin=2)
+            gi, _ = cs.bins(i)
+            assert np.array_equal(gi, ib), (L, n, i)
+            assert np.array_equal(cs.spins(i), spins.astype(np.int64)), (L, n, i)
