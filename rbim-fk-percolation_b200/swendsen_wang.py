@@ -150,6 +150,9 @@ class _SweepState:
         self.record, self.status = view("records", np.int32), view("status", np.int32)
         self.desc = view("chains", cs.desc_host.dtype)
         self.desc[:] = cs.desc_host
+        # The buffers are set up on this thread's stream; the next call may
+        # come from another thread on another one.
+        torch.cuda.current_stream(dev).synchronize()
 
     def run(self) -> None:
         """One sweep of the chain described by the host buffer; its spins, record and status come back there."""
