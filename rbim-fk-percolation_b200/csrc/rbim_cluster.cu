@@ -753,7 +753,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             // Tile cluster sizes minus one added onto each tile root's own index
             // (a root points at itself): afterwards the word of root m reads
             // m + size - 1, below 65536 because m is the smallest site of its tile
-            // cluster, so no add carries out of its 16 bits (tile_size decodes it).
+            // cluster, so no add carries out of its 16 bits (counted_size decodes it).
             // The likely largest tile cluster is counted by popcounts.
             cluster_count<NT>(x, tid);
             {
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                 const uint32_t hk = x.HK[k];
                 if (hk == kEmptyKey) continue;
                 const uint32_t m = node_key(hk), r = node_root(x, k);
-                const unsigned long long add = (unsigned long long)tile_size(u16, m) << 40 |
+                const unsigned long long add = (unsigned long long)counted_size(u16, m) << 40 |
                                                (unsigned long long)(m == likely ? red.likely_downs : hk >> 16) << 16;
                 atomicAdd(cl.map_shared_rank(x.HW, r >> 16) + (r & 0xFFFFu), add);
                 if (r == ((c << 16) | k)) ++nloc;
@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                     const uint32_t bb = __ffs(roots) - 1u;
                     roots &= roots - 1u;
                     const uint32_t m = (w << 5) + bb;
-                    top2_merge(k1, k2, size_key(tile_size(u16, m), tl.b + m), 0ull);
+                    top2_merge(k1, k2, size_key(counted_size(u16, m), tl.b + m), 0ull);
                 }
             }
             for (uint32_t k = tid; k < x.hs; k += NT) {
@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                         red.p_mc = (int)node_size(w) - 2 * (int)node_downs(w);
                         red.p_known = 1;
                     } else if (a1 && m == likely) {
-                        red.p_mc = (int)tile_size(u16, m) - 2 * (int)red.likely_downs;
+                        red.p_mc = (int)counted_size(u16, m) - 2 * (int)red.likely_downs;
                         red.p_known = 1;
                     }
                 }

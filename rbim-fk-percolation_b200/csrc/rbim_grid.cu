@@ -820,8 +820,8 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
             // Tile cluster sizes minus one added onto each tile root's own index
             // (a root points at itself): afterwards the word of root m reads
             // m + size - 1, below 65536 because m is the smallest site of its tile
-            // cluster, so no add carries out of its 16 bits (tile_size decodes it).
-            count_pieces<true>(t, u16, nullptr, warp, nwarps);
+            // cluster, so no add carries out of its 16 bits (counted_size decodes it).
+            count_pieces(t, u16, nullptr, warp, nwarps);
             __syncthreads();
             RBIM_GRID_MARK(12);
             // Node sizes into the root nodes' words (the high half of a root's
@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
                 if (k < nnodes) {
                     const uint32_t m = x.NK[k];
                     r = x.NR[k];
-                    v = tile_size(u16, m);
+                    v = counted_size(u16, m);
                     if (r == tl.b + m) ++nloc;
                 }
                 const uint32_t grp = __match_any_sync(0xFFFFFFFFu, r);
@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT) k_grid_sweeps(
                 const uint32_t bb = __ffs(roots) - 1u;
                 roots &= roots - 1u;
                 const uint32_t m = (w << 5) + bb;
-                top2_merge(k1, k2, size_key(tile_size(u16, m), tl.b + m), 0ull);
+                top2_merge(k1, k2, size_key(counted_size(u16, m), tl.b + m), 0ull);
             }
         }
         for (uint32_t k = tid; k < nnodes; k += NT) {

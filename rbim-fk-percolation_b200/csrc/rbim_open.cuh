@@ -360,8 +360,8 @@ __device__ __forceinline__ uint32_t piece_leaders(const Lat<Word16> &t, uint32_t
     return (head_mask(t.OV, w, valid) | 1u) & valid;
 }
 
-// Add v to the 16-bit word i through its 32-bit container (no carry can
-// leave the half: cluster sizes stay below 65536 whenever counts are taken).
+// Add v to the 16-bit word i through its 32-bit container.  The sum must stay
+// below 65536: a carry out of the low half would change the next site's word.
 __device__ __forceinline__ void add16(unsigned short *base, uint32_t i, uint32_t v)
 {
     atomicAdd((unsigned int *)(base + (i & ~1u)), v << (16u * (i & 1u)));
@@ -375,12 +375,10 @@ __device__ __forceinline__ void add16(unsigned short *base, uint32_t i, uint32_t
 // skip (or null): plane of the sites of one cluster, counted by popcounts
 // elsewhere; without it the largest cluster's root would take most of the
 // adds, one after the other.
-// kMinusOne: the piece that starts at the root adds one less, so that a root
-// word holds size - 1 (a tile of 65536 sites then still fits 16 bits).
-// Each root word must hold zero or the root's own index on entry (a root
-// points at itself, so counting onto it needs no zeroing pass; the caller
-// then subtracts the index).
-template <bool kMinusOne>
+// Each root m's word holds its own index on entry (a root points at itself, so
+// counting onto it needs no zeroing pass), and the piece that starts at the
+// root adds one less: the word ends as m + size - 1 (counted_size decodes it),
+// below 65536 since m is the smallest of its cluster's at most 65536 sites.
 __device__ __forceinline__ void count_pieces(const Lat<Word16> &t, unsigned short *u16, const uint32_t *skip,
                                              uint32_t warp, uint32_t nwarps)
 {
@@ -399,7 +397,7 @@ __device__ __forceinline__ void count_pieces(const Lat<Word16> &t, unsigned shor
                     const uint32_t n = (w << 5) + b;
                     const bool is_root = roots & bit;
                     const uint32_t r = is_root ? n : (uint32_t)u16[n];
-                    add16(u16, r, end - b - ((kMinusOne && is_root) ? 1u : 0u));
+                    add16(u16, r, end - b - (is_root ? 1u : 0u));
                 }
                 end = b;
             }
@@ -415,10 +413,16 @@ __device__ __forceinline__ void count_pieces(const Lat<Word16> &t, unsigned shor
                 const uint32_t end = next ? (uint32_t)(__ffs(next) - 1) : (uint32_t)__popc(valid);
                 const bool is_root = (t.ROOT[w] >> lane) & 1u;
                 const uint32_t r = is_root ? n : (uint32_t)u16[n];
-                add16(u16, r, end - lane - ((kMinusOne && is_root) ? 1u : 0u));
+                add16(u16, r, end - lane - (is_root ? 1u : 0u));
             }
         }
     }
+}
+
+// Size of the cluster of root m after count_pieces.
+__device__ __forceinline__ uint32_t counted_size(const unsigned short *u16, uint32_t m)
+{
+    return (((uint32_t)u16[m] - m) & 0xFFFFu) + 1u;
 }
 
 // The root most likely to have the largest cluster: of 32 sites spread over

@@ -475,11 +475,9 @@ __device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, u
         red.in_downs[warp] = in_downs;
     }
     RBIM_PHASE_MARK(6);
-    // Cluster sizes into the root words, on top of the index each root's word
-    // holds (a root points at itself): afterwards a root's word is root + size
-    // mod 2^16, which gives every size whenever there are two or more
-    // clusters (each then below 65536); one cluster is the lattice.
-    count_pieces<false>(t, u16, t.OH, warp, nwarps);
+    // Cluster sizes minus one into the root words, on top of the index each
+    // holds; the likely largest cluster is counted above.
+    count_pieces(t, u16, t.OH, warp, nwarps);
     __syncthreads();
     RBIM_PHASE_MARK(7);
     // Every warp sums the per-warp partials itself (no barrier needed after).
@@ -500,7 +498,7 @@ __device__ __forceinline__ void resident_measure(const Res &res, Red<NT> &red, u
                 const uint32_t b = __ffs(roots) - 1u;
                 roots &= roots - 1u;
                 const uint32_t r = (w << 5) + b;
-                const uint32_t size = r == likely ? in : ((uint32_t)u16[r] - r) & 0xFFFFu;
+                const uint32_t size = r == likely ? in : counted_size(u16, r);
                 top2_merge(k1, k2, (size << 16) | (0xFFFFu - r), 0u);
             }
         }

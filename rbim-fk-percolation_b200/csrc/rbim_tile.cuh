@@ -146,11 +146,4 @@ __device__ __forceinline__ uint32_t tile_root_walk(const unsigned short *uf, uin
     }
 }
 
-// Size of the tile cluster of tile root m once the sizes minus one have been
-// added onto the roots' own indices (count_pieces<true> without zeroing).
-__device__ __forceinline__ uint32_t tile_size(const unsigned short *u16, uint32_t m)
-{
-    return (((uint32_t)u16[m] - m) & 0xFFFFu) + 1u;
-}
-
 }  // namespace rbim
