@@ -87,6 +87,8 @@ def label_and_wrap_many(active: np.ndarray, L: int, device=None):
     if a.dtype == np.bool_:
         a = np.ascontiguousarray(a).view(np.uint8)  # a boolean is a byte of 0 or 1
     a = np.ascontiguousarray(a.reshape(-1, 2 * L * L), dtype=np.uint8)
+    if not a.flags.writeable:
+        a = a.copy()  # torch warns of a tensor over a read-only array (a frozen or memory-mapped mask)
     n = a.shape[0]
     lib = _native.lib()
     occ = torch.from_numpy(a).to(dev)
