@@ -199,7 +199,11 @@ def launch_buckets(lib, device, stream, launches: Sequence[Launch], *, spin_pool
 
 
 def require_cuda(device=None):
-    """Return the CUDA device to use; raise if there is none (no CPU fallback exists)."""
+    """Return the CUDA device to use, always with its index; raise if there is none (no CPU fallback exists).
+
+    ``"cuda"`` means the device that is current now: streams and state kept by device would otherwise follow the
+    caller's later choice of another one, away from the memory they belong to.
+    """
     torch = _torch()
     if not torch.cuda.is_available():
         raise _native.RbimError("the rbim B200 engine needs a CUDA device; none is available")
@@ -208,7 +212,7 @@ def require_cuda(device=None):
     d = torch.device(device)
     if d.type != "cuda":
         raise _native.RbimError(f"the rbim B200 engine runs on CUDA devices only, got {d}")
-    return d
+    return d if d.index is not None else torch.device("cuda", torch.cuda.current_device())
 
 
 def chain_key(seed) -> int:
