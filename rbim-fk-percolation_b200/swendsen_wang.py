@@ -119,9 +119,10 @@ def sw_sweep(spins: np.ndarray, lattice: Lattice, J: np.ndarray, beta: float, rn
 class _SweepState:
     """Device and host buffers of ``sw_sweep`` for L x L lattices on one device, used under ``lock``.
 
-    The chain set's inputs (bin sums, couplings, descriptor, spins) and its
-    outputs (spins, record, status) lie in one device buffer, mirrored in one
-    pinned host buffer, so that a call makes one copy in and one copy out.
+    The chain set's inputs (bin sums, couplings, descriptor, cleared status,
+    spins) and its outputs (status, spins, record) lie in one device buffer,
+    mirrored in one pinned host buffer, so that a call makes one copy in and
+    one copy out.
     """
 
     def __init__(self, L: int, dev):
@@ -133,7 +134,7 @@ class _SweepState:
         self.lock = threading.Lock()
         self.chain_set, self.device, self.threads = cs, dev, single_cta_threads(L)
         at, end = {}, 0
-        for name in ("acc_int", "acc_f64", "coupling_pool", "chains", "spin_pool", "records", "status"):
+        for name in ("acc_int", "acc_f64", "coupling_pool", "chains", "status", "spin_pool", "records"):
             t = getattr(cs, name)
             at[name] = (end, end + t.numel() * t.element_size())
             end = (at[name][1] + 15) & ~15
@@ -143,7 +144,7 @@ class _SweepState:
             t = getattr(cs, name)
             setattr(cs, name, device[lo:hi].view(t.dtype).view(t.shape))
         self._in = (device[: at["spin_pool"][1]], host[: at["spin_pool"][1]])
-        self._out = (device[at["spin_pool"][0]:], host[at["spin_pool"][0]:])
+        self._out = (device[at["status"][0]:], host[at["status"][0]:])
         h = host.numpy()
         view = lambda name, dtype: h[slice(*at[name])].view(dtype)  # noqa: E731
         self.couplings, self.spins = view("coupling_pool", "<u4"), view("spin_pool", "<u4")
@@ -157,6 +158,7 @@ class _SweepState:
     def run(self) -> None:
         """One sweep of the chain described by the host buffer; its spins, record and status come back there."""
         cs, stream = self.chain_set, _torch().cuda.current_stream(self.device)
+        self.status[0] = 0  # the kernels only add bits: an earlier call's error is not this one's
         try:
             self._in[0].copy_(self._in[1], non_blocking=True)
             if self.engine == "grid":
