@@ -50,6 +50,14 @@ constexpr uint32_t kTileHalf = 32768;   // tiles of the 512-thread mode
 constexpr uint32_t kClusterMax = 16;    // non-portable cluster size limit
 constexpr uint32_t kHashMax = 4096;     // node slots per tile (12 bits of a node id)
 constexpr uint32_t kEmptyKey = 0xFFFFFFFFu;
+
+// Where the probe for key m starts in a node table of hs slots, and the slot
+// after h.  The last slot is never used: a hash word also holds root node <<
+// 16 | key for a while, and root node (tile 15, slot 4095) with key 65535
+// would read as an empty slot.
+__device__ __forceinline__ uint32_t node_probe(uint32_t m, uint32_t hs) { return __umulhi(m * 0x9E3779B1u, hs - 1u); }
+__device__ __forceinline__ uint32_t node_next(uint32_t h, uint32_t hs) { return h + 2u < hs ? h + 1u : 0u; }
+
 constexpr size_t kSmemBudget = 227 * 1024 - 4 * 1024;  // one CTA per SM
 constexpr size_t kSmemPerSm = 228 * 1024;
 constexpr size_t kStaticSmem = 2 * 1024;
@@ -68,7 +76,7 @@ __host__ __device__ constexpr uint32_t cluster_hash_size(uint32_t l_max, uint32_
     const uint32_t rows = T / l_max + 2u;
     const uint32_t bound = 2u * l_max + 2u * rows + 1u;
     uint32_t h = 64;
-    while (h < bound + bound / 4u) h *= 2;
+    while (h < bound + bound / 4u) h *= 2;  // one slot stays empty (node_probe)
     return h;
 }
 
@@ -180,7 +188,7 @@ struct Ctx {
     uint32_t *YS;
     uint32_t *HK;
     unsigned long long *HW;
-    uint32_t hs, hs_log2;
+    uint32_t hs;
 };
 
 __device__ __forceinline__ Ctx make_ctx(unsigned char *smem, const ClusterLayout &ly, const Tile &tl, CRed &red)
@@ -208,7 +216,6 @@ __device__ __forceinline__ Ctx make_ctx(unsigned char *smem, const ClusterLayout
     x.HK = (uint32_t *)(smem + ly.off_HK);
     x.HW = (unsigned long long *)(smem + ly.off_HW);
     x.hs = ly.hs;
-    x.hs_log2 = 31u - __clz(ly.hs);
     return x;
 }
 
@@ -221,7 +228,7 @@ struct Dist {
     cg::cluster_group cl;
     uint32_t *HK;
     unsigned long long *HW;
-    uint32_t hs, hs_log2;
+    uint32_t hs;
     int *wrap, *err;
     uint32_t cap;
 
@@ -247,11 +254,11 @@ struct Dist {
     __device__ __forceinline__ uint32_t insert(uint32_t tile, uint32_t m) const
     {
         uint32_t *hk = cl.map_shared_rank(HK, tile);
-        uint32_t h = (m * 0x9E3779B1u) >> (32u - hs_log2);
+        uint32_t h = node_probe(m, hs);
         for (uint32_t it = 0; it < hs; ++it) {
             const uint32_t old = atomicCAS(hk + h, kEmptyKey, m);
             if (old == kEmptyKey || old == m) return (tile << 16) | h;
-            h = (h + 1u) & (hs - 1u);
+            h = node_next(h, hs);
         }
         atomicOr(err, kErrUnionCap);
         return (tile << 16) | 0u;
@@ -465,8 +472,8 @@ __device__ __forceinline__ uint32_t node_size(unsigned long long w) { return (ui
 // passes before is taken, so the first whose key's low half is m is its own.
 __device__ __forceinline__ uint32_t node_slot(const Ctx &x, uint32_t m)
 {
-    uint32_t h = (m * 0x9E3779B1u) >> (32u - x.hs_log2);
-    for (uint32_t it = 0; it < x.hs && (x.HK[h] & 0xFFFFu) != m; ++it) h = (h + 1u) & (x.hs - 1u);
+    uint32_t h = node_probe(m, x.hs);
+    for (uint32_t it = 0; it < x.hs && (x.HK[h] & 0xFFFFu) != m; ++it) h = node_next(h, x.hs);
     return h;
 }
 
@@ -648,7 +655,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
         tl.inv = tile_inv(tl.L);
         const Ctx x = make_ctx(smem, ly, tl, red);
         const Lat<Word16> &t = x.t;
-        const Dist d{cl, x.HK, x.HW, x.hs, x.hs_log2, &red.wrap, &red.err, C * x.hs + 64u};
+        const Dist d{cl, x.HK, x.HW, x.hs, &red.wrap, &red.err, C * x.hs + 64u};
         uint32_t *gS = spin_pool + ch.spin_off + (tl.b >> 5);
         const uint32_t *gJH = coupling_pool + ch.coupling_off + (tl.b >> 5);
         const uint32_t *gJV = coupling_pool + ch.coupling_off + tl.nwp + (tl.b >> 5);
