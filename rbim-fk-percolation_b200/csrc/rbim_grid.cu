@@ -587,9 +587,12 @@ __device__ __forceinline__ void grid_boundary(const GTile &x, const Tile &tl, co
         // The first bond into a node of the next tile hooks it under this
         // tile's node, without a walk: the tree of a root rb > ra holds only
         // nodes from rb on, so ra cannot be in it.  (One L = 249 lattice 35.8
-        // -> 34.4 us a sweep; hooking only every other tile, for shallower
-        // trees, 34.6.)
-        if (live && !(ex | ey) && rb > ra && rb < tl.N) {
+        // -> 34.4 us a sweep.)  Not from every sixteenth tile: where each tile
+        // has one cluster and its rows begin with it, no other bond walks, and
+        // the nodes would stay a chain of all tiles, which every tile then
+        // follows (L = 1024 ordered 81 us a sweep, this way 37, L = 256 40 and
+        // 23; costs 0.5 % at T >= 1, every eighth or fourth tile up to 3 %).
+        if (live && (tl.c & 15u) != 15u && !(ex | ey) && rb > ra && rb < tl.N) {
             const unsigned long long self = Word64::make(rb, 0, 0);
             if (atomicCAS(ws.G + rb, self, Word64::make(ra, 0, 0)) == self) live = false;
         }
