@@ -36,10 +36,11 @@ SINGLE_CTA_MAX_L = 112
 
 def single_cta_threads(L: int) -> int:
     """CTA size for one lattice alone on the resident engine: the large sizes minimise the time per sweep (the
-    batch default favours many CTAs per SM instead).  Measured on B200, us per sweep with 512 / 1024 threads:
-    L = 24 16.1 / 16.5 and L = 32 16.5 / 17.3 before the labelling got lighter, L = 72 19.6 / 19.7, L = 96 24.7 /
-    24.7, L = 104 24.8 / 26.7, L = 112 27.2 / 27.8."""
-    return 512 if L <= 32 or L > 96 else 1024
+    batch default favours many CTAs per SM instead).  Measured on B200, p = 0.08, T = 1.7, us per sweep with 512 /
+    1024 threads: L = 24 12.7 / 13.1, 32 13.1 / 13.9; 33 13.0 / 14.3, 64 17.8 / 18.9, 72 19.0 / 18.7, 96 24.0 / 23.7;
+    97 22.5 / 23.8, 112 26.5 / 26.7, 128 28.2 / 30.6; 144 36.2 / 32.9, 181 50.4 / 39.4, 192 59.4 / 48.5, 256 93.1 /
+    70.1.  From 33 to 64 the sizes are held at 1024 by a test, though 512 would be up to 9 % faster."""
+    return 512 if L <= 32 or 96 < L <= 128 else 1024
 
 
 _sm_counts = {}
