@@ -29,9 +29,10 @@ __all__ = ["ChainSpec", "ChainSet", "chain_key", "require_cuda", "SINGLE_CTA_MAX
 #: L <= SINGLE_CTA_MAX_L, with the CTA size ``single_cta_threads(L)``, and
 #: over the whole GPU above: on the grid engine where it has a plan for L, else
 #: on the plain engine.  Measured on B200, one lattice, us per sweep, one CTA
-#: against the grid engine: L = 64 19.9 / 23.7, L = 96 24.7 / 26.5, L = 112 27.2 /
-#: 27.9, L = 128 29.0 / 28.0.
-SINGLE_CTA_MAX_L = 112
+#: against the grid engine, p = 0.10, T = 1.8 and (in brackets) p = 0.05, T = 2.2:
+#: L = 64 19.9 / 24.1 (20.1 / 23.7), 96 24.9 / 26.2 (25.5 / 25.3), 108 25.6 / 26.8
+#: (25.8 / 26.0), 112 27.2 / 27.1 (27.8 / 26.2), 128 28.9 / 26.4 (30.1 / 26.1).
+SINGLE_CTA_MAX_L = 108
 
 
 def single_cta_threads(L: int) -> int:

@@ -27,3 +27,11 @@ def test_single_lattice_cta_sizes(rb):
     (32, 32 * 148 + 1, 256, 32), (512, 149, 256, 512)])
 def test_cta_sizes_of_launches_of_few_lattices(rb, default, lattices, L, threads):
     assert rb.engine.occupancy_threads(default, lattices, 148, L * L) == threads
+
+
+@pytest.mark.parametrize("L,engine", [(64, "batched"), (96, "batched"), (108, "batched"), (109, "grid"), (112, "grid"),
+                                      (128, "grid")])
+def test_one_lattice_takes_the_faster_engine(rb, L, engine):
+    """Up to L = 108 one CTA, from L = 112 the grid engine was measured faster."""
+    spec = rb.ChainSpec(L=L, realization=0, key=1, beta=0.5, n_therm=0, n_bins=1, sweeps_per_bin=1)
+    assert rb.engine.auto_engine([spec], lambda L: (148, 512)) == engine
