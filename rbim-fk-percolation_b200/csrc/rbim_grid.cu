@@ -590,8 +590,9 @@ __device__ __forceinline__ void grid_boundary(const GTile &x, const Tile &tl, co
         // -> 34.4 us a sweep.)  Not from every sixteenth tile: where each tile
         // has one cluster and its rows begin with it, no other bond walks, and
         // the nodes would stay a chain of all tiles, which every tile then
-        // follows (L = 1024 ordered 81 us a sweep, this way 37, L = 256 40 and
-        // 23; costs 0.5 % at T >= 1, every eighth or fourth tile up to 3 %).
+        // follows (without an open bond L = 1024 took 80 us a sweep, this way
+        // 38 to 41, L = 256 40 and 23; costs 0.5 % at T >= 1, every eighth or
+        // fourth tile up to 3 %).
         if (live && (tl.c & 15u) != 15u && !(ex | ey) && rb > ra && rb < tl.N) {
             const unsigned long long self = Word64::make(rb, 0, 0);
             if (atomicCAS(ws.G + rb, self, Word64::make(ra, 0, 0)) == self) live = false;
@@ -1117,10 +1118,14 @@ GridPlan grid_plan(uint32_t L)
     // larger ones add walk latency inside the tile), at most one per SM; then
     // the largest tile count at or below that whose tiles all hold at least L
     // sites.  512 threads for tiles of up to 1024 sites, else 1024.  Measured
-    // on B200, one lattice, us per sweep: L = 128: 16 x 512 28.0, 16 x 1024
-    // 29.1, 32 x 512 27.6, 8 x 512 28.7; L = 249: 61 x 512 32.0, 61 x 1024 32.8,
-    // 20 x 512 34.7; L = 512: 128 x 1024 37.7, 128 x 512 38.7, 74 x 1024 39.6;
-    // L = 1024: 128 x 1024 50.5, 128 x 512 55.7, 74 x 1024 57.7.
+    // on B200, one lattice, us per sweep, the plan taken first: L = 128: 16 x
+    // 512 26.5; 16 x 1024 27.0, 32 x 512 26.7, 8 x 512 26.4; L = 200: 35 x 1024
+    // 30.8; 32 x 512 29.4, 20 x 512 29.7; L = 249: 61 x 512 30.8; 61 x 1024
+    // 31.2, 31 x 512 31.8; L = 256: 64 x 512 31.0; 128 x 512 30.9, 32 x 512
+    // 31.1; L = 512: 147 x 1024 37.0; 128 x 1024 36.2, 147 x 512 38.6, 74 x 1024
+    // 37.6; L = 1024: 147 x 1024 48.2; 128 x 1024 47.8, 147 x 512 52.1, 74 x
+    // 1024 53.6; L = 2048: 148 x 1024 82.3; 128 x 1024 83.2, 148 x 512 99.2.
+    // Where another plan is faster it is so by 2 %, at L = 200 by 5 %.
     const int sms = device_sm_count();
     if (sms <= 0) return {0u, 0u};
     const uint64_t want = ((uint64_t)L * L + 1023u) / 1024u;

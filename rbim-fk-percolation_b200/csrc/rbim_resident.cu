@@ -127,9 +127,11 @@ __host__ __device__ constexpr ResidentLayout resident_layout_c(uint32_t l_max, i
     ly.off_ROOT = off;
     off += plane;
     // Row-end masks, for the CTA sizes of the small lattices: several rows end
-    // in a word there (masks computed each sweep cost 3 % at L = 64, 10 % at
-    // L = 40). Larger CTAs compute them: without the plane a fourth CTA of 256
-    // threads fits an SM at L = 127 and 128 (-8 %).
+    // in a word there (16384 lattices, us a sweep with the plane / with masks
+    // computed by the reciprocal: L = 32 207 / 211, 44 398 / 404, 64 588 / 592,
+    // 40 365 / 366, 16, 24, 48 and 56 the same). Larger CTAs compute them:
+    // without the plane a fourth CTA of 256 threads fits an SM at L = 127 and
+    // 128 (-8 %).
     ly.off_RE = off;
     if (threads <= 128) off += plane;
     ly.off_SEAMV = off;

@@ -619,9 +619,9 @@ class ChainSet:
         L <= SINGLE_CTA_MAX_L on one resident CTA of ``single_cta_threads(L)``
         threads, one larger lattice over the whole GPU -- on the grid engine
         where it has a plan, else on the plain engine -- and any other set on
-        the batched engines.  On B200 a sweep of one L = 256 lattice takes 32 us
-        on the grid engine, 56 us on the plain engine and 75 us on one resident
-        CTA; L = 1024 50 us, 160 us and 115 us on one 16-CTA cluster.
+        the batched engines.  On B200 a sweep of one L = 256 lattice takes 31 us
+        on the grid engine, 52 us on the plain engine and 73 us on one resident
+        CTA; L = 1024 48 us, 160 us and 106 us on one 16-CTA cluster.
         Results are the same on every engine.
         """
         if engine == "auto":
