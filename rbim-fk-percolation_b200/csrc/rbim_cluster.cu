@@ -173,7 +173,7 @@ struct CRed {
     int pass;
     // Per chain / per sweep state.
     int item, wrap, err;
-    uint32_t likely_downs;
+    uint32_t heads, likely_downs;
     uint32_t front, tile_end;
     Acc acc;
     long long cur_bin;
@@ -517,9 +517,52 @@ static __device__ __noinline__ void cluster_count(const Ctx &x, uint32_t tid)
 }
 
 template <int NT>
-static __device__ __noinline__ void cluster_heads(const Lat<Word16> &t, uint32_t warp)
+static __device__ __noinline__ void cluster_heads(const Lat<Word16> &t, uint32_t warp, uint32_t *total)
 {
-    phase_heads_open<false>(t, warp, NT / 32);
+    phase_heads_open<false, true>(t, warp, NT / 32, total);
+}
+
+// Roots and flip of a tile with few run heads (an ordered lattice at low
+// temperature): one lane per word and one walk per run piece, whose first site
+// alone gets its root (the measurement reads no other).  The walk of a word
+// inside a run starts at the last site of the nearest word before it, in the
+// warp's 32, that has a head.  roots_flip_sites takes the same time for every
+// lattice; this pass goes by runs.
+template <int NT>
+static __device__ __noinline__ void cluster_roots_runs(const Lat<Word16> &t, uint32_t *in, uint32_t root, uint32_t warp)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t w0 = warp << 5; w0 < t.g.NW; w0 += NT) {
+        const uint32_t w = w0 + lane;
+        const uint32_t valid = w < t.g.NW ? t.g.valid(w) : 0u;
+        const uint32_t heads = valid ? head_mask(t.OV, w, valid) : 0u;
+        const uint32_t headed = __ballot_sync(0xFFFFFFFFu, heads != 0u) & (mask_le(lane) >> 1);
+        uint32_t roots = 0, flips = 0, members = 0, left = valid, cut = (heads | 1u) & valid;
+        while (cut) {
+            const uint32_t b = 31u - __clz(cut), bit = 1u << b, pm = left & (0u - bit), n = (w << 5) + b;
+            cut ^= bit;
+            left ^= pm;
+            uint32_t r = t.uf.ld(heads & bit ? n : ((w0 + 32u - __clz(headed)) << 5) - 1u);
+            for (uint32_t it = 0;; ++it) {
+                const uint32_t p = t.uf.ld(r);
+                r = t.uf.ld(p);
+                if (p == r) break;
+                if (it >= t.cap) {
+                    atomicOr(t.err, kErrFindCap);
+                    break;
+                }
+            }
+            t.uf.st(n, (unsigned short)r);
+            if (r == n) roots |= bit;
+            if ((t.FLIP[r >> 5] >> (r & 31u)) & 1u) flips |= pm;
+            if (r == root) members |= pm;
+        }
+        if (w < t.g.NW) {
+            t.ROOT[w] = roots;
+            t.S[w] ^= flips;
+            if (in) in[w] = members;
+        }
+    }
 }
 
 // The magnetizations of this tile's parts of the largest and (second) the
@@ -676,6 +719,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             if (tid == 0) {
                 red.wrap = 0;
                 red.tile_end = 0;
+                red.heads = 0;
             }
             for (uint32_t i = tid; i < 16u; i += NT) x.YS[i] = 0u;
             __syncthreads();
@@ -683,9 +727,9 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
                               nwarps, tid);
             __syncthreads();
             if constexpr (CC == 16)
-                cluster_heads<NT>(t, warp);
+                cluster_heads<NT>(t, warp, &red.heads);
             else
-                phase_heads_open<false>(t, warp, nwarps);
+                phase_heads_open<false, true>(t, warp, nwarps, &red.heads);
             for (uint32_t k = tid; k < x.hs; k += NT) x.HK[k] = kEmptyKey;
             __syncthreads();
             // The warp's union list lies in its share of the node words, which
@@ -733,8 +777,25 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 1024 / NT)
             // Tile roots, ROOT bits and flip; in measured sweeps the sites of
             // the tile cluster most likely to be its largest go to the OH
             // plane, which is free until the next activation.
-            const uint32_t likely = measure ? likely_largest(t) : 0u;
-            roots_flip_sites<true, 4>(t, measure ? t.OH : nullptr, likely, warp, nwarps);
+            //
+            // By runs below two run heads a word: roots_flip_sites takes 37 k
+            // cycles at L = 512 whatever the lattice, cluster_roots_runs 12 k
+            // without an open bond, and the more the more runs there are.  B200,
+            // us a sweep by sites / by runs, p = 0: L = 512 (33 lattices) T =
+            // 0.02 73.2 / 46.2, 0.4 77.2 / 60.3, 0.7 77.6 / 66.4 (2 heads a
+            // word), 0.8 79.1 / 73.6; L = 1024 (8) 162 / 110, 157 / 126, 160 /
+            // 142, 164 / 165.  With four heads a word the runs lose (L = 1024, p =
+            // 0.1, T = 0.5 168 / 179).  A tile that goes by runs takes the
+            // cluster of its middle site for the likely largest: the 32 walks of
+            // likely_largest pass row heads that lie in one bank (21 k cycles).
+            uint32_t likely = 0;
+            if (red.heads < 2u * t.g.NW) {
+                if (measure) likely = uf_root_ro<Word16>(t.uf, (t.g.N + tl.L) >> 1, t.cap, t.err);
+                cluster_roots_runs<NT>(t, measure ? t.OH : nullptr, likely, warp);
+            } else {
+                if (measure) likely = likely_largest(t);
+                roots_flip_sites<true, 4>(t, measure ? t.OH : nullptr, likely, warp, nwarps);
+            }
             __syncthreads();
             cl.sync();  // every flip is done
             tile_halo<NT>(x, tl, cl, red, tid);

@@ -171,9 +171,10 @@ __device__ __forceinline__ uint32_t open_parent(const UF<Word16> &uf, const UpBo
 // Per group of 32 words, lane j finds the heads and up-bonds of word j.  Bound
 // by the integer pipe, so what can be done on whole words is done there.  kFew:
 // for launches whose warps may have a single word, which all lanes then look
-// at.
-template <bool kFew>
-__device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t warp, uint32_t nwarps)
+// at.  kCount: the number of heads is added to *total.
+template <bool kFew, bool kCount = false>
+__device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t warp, uint32_t nwarps,
+                                                 uint32_t *total = nullptr)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const Geom &g = t.g;
@@ -187,6 +188,7 @@ __device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t 
         return;
     }
     const uint32_t band0 = band.first << 5, b0 = 2u * (lane & 15u), le0 = mask_le(b0), le1 = 2u * le0 + 1u;
+    uint32_t heads = 0;
     for (uint32_t base = band.first; base < band.end; base += 32u) {
         const uint32_t wj = base + lane;
         UpBonds ub{};
@@ -194,6 +196,7 @@ __device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t 
             ub = up_bonds(t, wj);
             t.NEED[wj] = ub.need;
         }
+        if (kCount) heads += __popc(ub.heads);
         const uint32_t count = min(32u, band.end - base);
         for (uint32_t j = 0; j < count; j += 2u) {
             const uint32_t jj = j + (lane >> 4);
@@ -214,6 +217,10 @@ __device__ __forceinline__ void phase_heads_open(const Lat<Word16> &t, uint32_t 
             }
             __syncwarp();  // later rows read these words
         }
+    }
+    if (kCount) {
+        heads = __reduce_add_sync(0xFFFFFFFFu, heads);
+        if (lane == 0) atomicAdd(total, heads);
     }
 }
 
